@@ -1627,9 +1627,14 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
       SIH26_TEAM_MARK(5);
       --evaluations;
       if (resident && c.state == kRunning) {
-        if (kDelta<T> && ts.flags[1]) load_vectors(P, S, pl, c.cur);
+        const bool refill = kDelta<T> && ts.flags[1] != 0;  // the same in every block
+        if (refill) load_vectors(P, S, pl, c.cur);
         if (ts.flags[1] || !halpern) load_epilogues(P, S, sp, sd, halpern, c.cur);
-        __syncthreads();
+        // The Halpern operator's next step stores into every block's only copy of x: not before they have all
+        // been refilled, or a block that is behind writes the restart's zeros over a new entry. Some 500
+        // cycles a restart.
+        if (refill) tm.sync();
+        else __syncthreads();
       }
     }
   }
