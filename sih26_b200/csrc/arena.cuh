@@ -5,7 +5,6 @@
 #include <cstring>
 #include <memory>
 #include <string>
-#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -38,8 +37,8 @@ class Arena {
     // whatever ended the call, nothing may still be using the chunks when they are kept
     const bool idle = cudaStreamSynchronize(stream_) == cudaSuccess;
     for (const auto& c : chunks_) {
-      if (idle) MemoryCache::get().give_device(device_, c.first, c.second);
-      else cudaFree(c.first);
+      if (idle) MemoryCache::get().give_device(c);
+      else cudaFree(c.p);
     }
   }
   template <class T>
@@ -49,12 +48,11 @@ class Arena {
     if (bytes > left_) {
       end_range();
       constexpr size_t kChunk = size_t(64) << 20;
-      size_t size = 0;
-      void* p = MemoryCache::get().take_device(device_, std::max(bytes, kChunk), &size);
-      if (!p) throw Failure{SANKHYA_GPU_OUT_OF_MEMORY, "cudaMalloc: out of memory"};
-      chunks_.emplace_back(p, size);
-      next_ = static_cast<unsigned char*>(p);
-      left_ = size;
+      const Chunk c = MemoryCache::get().take_device(device_, std::max(bytes, kChunk));
+      if (!c) throw Failure{SANKHYA_GPU_OUT_OF_MEMORY, "cudaMalloc: out of memory"};
+      chunks_.push_back(c);
+      next_ = static_cast<unsigned char*>(c.p);
+      left_ = c.bytes;
       range_ = next_;
     }
     void* p = next_;
@@ -136,7 +134,7 @@ class Arena {
       SIH26_CUDA(cudaMemsetAsync(range_, 0, next_ - range_, stream_), SANKHYA_GPU_COPY_FAILED);
     range_ = next_;
   }
-  std::vector<std::pair<void*, size_t>> chunks_;
+  std::vector<Chunk> chunks_;
   unsigned char* next_ = nullptr;
   size_t left_ = 0;
   int device_ = 0;

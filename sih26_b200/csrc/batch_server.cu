@@ -96,8 +96,7 @@ struct Job {
   int slot = -1;
   unsigned char* base = nullptr;  // its device region: in the pool at pool_offset, or
   size_t pool_offset = 0;
-  void* own_chunk = nullptr;      // a chunk of its own
-  size_t own_chunk_bytes = 0;
+  Chunk own_chunk;                // a chunk of its own
   bool finished = false;
   bool model_error = false;
   std::string message;
@@ -381,8 +380,7 @@ struct Server {
   unsigned char* pool = nullptr;
   size_t pool_bytes = 0;  // what the LPs may take
   // the chunks of the memory cache that everything below sits in
-  void *device_chunk = nullptr, *pinned_chunk = nullptr, *table_chunk = nullptr;
-  size_t device_chunk_bytes = 0, pinned_chunk_bytes = 0, table_chunk_bytes = 0;
+  Chunk device_chunk, pinned_chunk, table_chunk;
   std::unique_ptr<PoolAllocator> alloc;
   BatchSlot* d_slots = nullptr;
   NewSlot* d_fresh = nullptr;  // the LPs being admitted
@@ -802,8 +800,8 @@ static void solve_one_solo(Server& s) {
 
 static void release(Server& s, Job& J) {
   if (J.own_chunk) {
-    MemoryCache::get().give_device(s.cfg.device, J.own_chunk, J.own_chunk_bytes);
-    J.own_chunk = nullptr;
+    MemoryCache::get().give_device(J.own_chunk);
+    J.own_chunk = Chunk{};
   } else if (J.base) {
     s.alloc->release(J.pool_offset, J.bytes);
   }
@@ -819,8 +817,8 @@ static void admit(Server& s) {
     size_t at = 0;
     if (J->bytes > s.pool_bytes) {
       // larger than the whole pool by its slices and scratch only: a chunk of its own
-      J->own_chunk = MemoryCache::get().take_device(s.cfg.device, J->bytes, &J->own_chunk_bytes);
-      J->base = static_cast<unsigned char*>(J->own_chunk);
+      J->own_chunk = MemoryCache::get().take_device(s.cfg.device, J->bytes);
+      J->base = static_cast<unsigned char*>(J->own_chunk.p);
       if (!J->base) {
         s.waiting.pop_front();
         J->status = SANKHYA_PDHG_NUMERICAL_ERROR;
@@ -1050,20 +1048,20 @@ int sankhya_pdhg_server_create(const sankhya_pdhg_server_config* config,
                                           : share;
     s->pool_bytes &= ~size_t(255);
     // one chunk each for the LPs, the device tables and the pinned mirrors
-    const auto chunk = [&](size_t bytes, size_t* got) {
-      void* p = cache.take_device(s->cfg.device, std::max<size_t>(bytes, 256), got);
-      if (!p) throw Failure{SANKHYA_GPU_OUT_OF_MEMORY, "cudaMalloc: out of memory"};
-      return p;
+    const auto chunk = [&](size_t bytes) {
+      const sih26::Chunk c = cache.take_device(s->cfg.device, std::max<size_t>(bytes, 256));
+      if (!c) throw Failure{SANKHYA_GPU_OUT_OF_MEMORY, "cudaMalloc: out of memory"};
+      return c;
     };
-    s->device_chunk = chunk(s->pool_bytes, &s->device_chunk_bytes);
-    s->pool = static_cast<unsigned char*>(s->device_chunk);
+    s->device_chunk = chunk(s->pool_bytes);
+    s->pool = static_cast<unsigned char*>(s->device_chunk.p);
     s->alloc = std::make_unique<sih26::PoolAllocator>(s->pool_bytes);
     const size_t slots_b = (cap * sizeof(sih26::BatchSlot) + 255) & ~size_t(255);
     const size_t ctrls_b = (cap * sizeof(sih26::Ctrl) + 255) & ~size_t(255);
     const size_t list_b = (cap * sizeof(int) + 255) & ~size_t(255);
     const size_t fresh_b = (cap * sizeof(sih26::NewSlot) + 255) & ~size_t(255);
-    s->table_chunk = chunk(slots_b + fresh_b + 3 * ctrls_b + 2 * (list_b + 512) + 256, &s->table_chunk_bytes);
-    unsigned char* at = static_cast<unsigned char*>(s->table_chunk);
+    s->table_chunk = chunk(slots_b + fresh_b + 3 * ctrls_b + 2 * (list_b + 512) + 256);
+    unsigned char* at = static_cast<unsigned char*>(s->table_chunk.p);
     const auto carve = [&](size_t bytes) {
       unsigned char* p = at;
       at += bytes;
@@ -1081,9 +1079,9 @@ int sankhya_pdhg_server_create(const sankhya_pdhg_server_config* config,
       SIH26_SCUDA(cudaMemsetAsync(s->d_count[k], 0, sizeof(int), s->stream), SANKHYA_GPU_INIT_FAILED);
     }
     unsigned long long* d_clock = reinterpret_cast<unsigned long long*>(carve(256));
-    s->pinned_chunk = cache.take_pinned(2 * ctrls_b + 2 * list_b + 256, &s->pinned_chunk_bytes);
+    s->pinned_chunk = cache.take_pinned(2 * ctrls_b + 2 * list_b + 256);
     if (!s->pinned_chunk) throw Failure{SANKHYA_GPU_OUT_OF_MEMORY, "cudaMallocHost: out of memory"};
-    at = static_cast<unsigned char*>(s->pinned_chunk);
+    at = static_cast<unsigned char*>(s->pinned_chunk.p);
     s->h_compact = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
     s->h_compact2 = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
     s->h_active = reinterpret_cast<int*>(carve(list_b));
@@ -1115,19 +1113,16 @@ void sankhya_pdhg_server_free(sankhya_pdhg_server* server) {
   const bool idle = !s->stream || cudaStreamSynchronize(s->stream) == cudaSuccess;
   if (s->graph) cudaGraphExecDestroy(s->graph);
   sih26::MemoryCache& cache = sih26::MemoryCache::get();
-  const auto back = [&](void* p, size_t bytes) {
-    if (!p) return;
-    if (idle) cache.give_device(s->cfg.device, p, bytes);
-    else cudaFree(p);
+  const auto back = [&](const sih26::Chunk& c) {
+    if (idle) cache.give_device(c);
+    else if (c) cudaFree(c.p);
   };
-  back(s->device_chunk, s->device_chunk_bytes);
-  back(s->table_chunk, s->table_chunk_bytes);
-  if (s->pinned_chunk) {
-    if (idle) cache.give_pinned(s->pinned_chunk, s->pinned_chunk_bytes);
-    else cudaFreeHost(s->pinned_chunk);
-  }
+  back(s->device_chunk);
+  back(s->table_chunk);
+  if (idle) cache.give_pinned(s->pinned_chunk);
+  else if (s->pinned_chunk) cudaFreeHost(s->pinned_chunk.p);
   for (auto& J : s->slot_job)
-    if (J && J->own_chunk) back(J->own_chunk, J->own_chunk_bytes);
+    if (J) back(J->own_chunk);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
 }
