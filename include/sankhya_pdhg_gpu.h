@@ -402,6 +402,13 @@ int sankhya_pdhg_wire_view(const void* buffer, size_t bytes, sankhya_pdhg_proble
 /* Reason for the most recent failing call on this thread (never NULL). */
 const char* sankhya_pdhg_gpu_last_error(void);
 
+/* Between calls the library keeps device memory that a solve, a batch or a freed server has finished
+ * with, up to 2 GiB a device, and up to 64 MiB of pinned host memory, for the next call: an allocation of its
+ * own that fails gives it back by itself, another allocator's does not. This call gives it back for `device`
+ * (thread-safe; memory in use by calls and servers stays theirs); *released, unless NULL, gets the bytes
+ * of device memory freed. cudaDeviceReset while a call runs or a server is open is not supported. */
+int sankhya_pdhg_gpu_release_memory(int device, int64_t* released);
+
 /* Device queries, the successors of is_cuda_available / get_gpu_device_count
  * (include/sankhya/gpu_runtime.hpp:71-77). */
 int sankhya_pdhg_gpu_device_count(void);

@@ -1627,6 +1627,24 @@ int sankhya_pdhg_gpu_device_count(void) {
   return n;
 }
 
+int sankhya_pdhg_gpu_release_memory(int device, int64_t* released) {
+  if (released) *released = 0;
+  int devices = 0;
+  if (cudaGetDeviceCount(&devices) != cudaSuccess || devices == 0) {
+    cudaGetLastError();
+    sih26::g_last_error = "no CUDA device is visible";
+    return SANKHYA_GPU_NO_COMPATIBLE_DEVICE;
+  }
+  if (device < 0 || device >= devices) {
+    sih26::g_last_error = "device ordinal out of range";
+    return SANKHYA_GPU_INVALID_ARGUMENT;
+  }
+  sih26::DeviceGuard guard;
+  const size_t bytes = sih26::MemoryCache::get().release(device);
+  if (released) *released = static_cast<int64_t>(bytes);
+  return SANKHYA_GPU_SUCCESS;
+}
+
 int sankhya_pdhg_gpu_device_name(int device, char* name, int capacity) {
   cudaDeviceProp p{};
   if (cudaGetDeviceProperties(&p, device) != cudaSuccess) {

@@ -109,7 +109,8 @@ class _Result(C.Structure):
 # Every symbol include/sankhya_pdhg_gpu.h declares.
 EXPORTED_SYMBOLS = ("sankhya_pdhg_gpu_default_params", "sankhya_pdhg_gpu_solve",
                     "sankhya_pdhg_gpu_last_error", "sankhya_pdhg_gpu_device_count",
-                    "sankhya_pdhg_gpu_device_name", "sankhya_pdhg_gpu_residuals_noalloc",
+                    "sankhya_pdhg_gpu_device_name", "sankhya_pdhg_gpu_release_memory",
+                    "sankhya_pdhg_gpu_residuals_noalloc",
                     "sankhya_pdhg_server_default_config", "sankhya_pdhg_server_create",
                     "sankhya_pdhg_server_submit", "sankhya_pdhg_server_step",
                     "sankhya_pdhg_server_result", "sankhya_pdhg_server_free",
@@ -136,12 +137,24 @@ def load_library() -> C.CDLL:
                                                C.POINTER(_Result)]
         lib.sankhya_pdhg_gpu_last_error.restype = C.c_char_p
         lib.sankhya_pdhg_gpu_device_name.argtypes = [C.c_int, C.c_char_p, C.c_int]
+        lib.sankhya_pdhg_gpu_release_memory.argtypes = [C.c_int, C.POINTER(C.c_int64)]
         _lib = lib
     return _lib
 
 
 def device_count() -> int:
     return load_library().sankhya_pdhg_gpu_device_count()
+
+
+def release_memory(device: int = 0) -> int:
+    """Gives back the device and pinned host memory the library keeps between calls (up to 2 GiB and
+    64 MiB a device); returns the bytes of device memory freed."""
+    lib = load_library()
+    freed = C.c_int64(0)
+    code = lib.sankhya_pdhg_gpu_release_memory(device, C.byref(freed))
+    if code != 0:
+        raise GpuError(code, lib.sankhya_pdhg_gpu_last_error().decode())
+    return freed.value
 
 
 class Options:
