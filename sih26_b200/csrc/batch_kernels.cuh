@@ -5,10 +5,10 @@
 // src/pdhg/pdhg.cpp:267-726 on one LP: the norm estimate, the attempts, the evaluations every 40
 // accepted iterations with per-LP restarts and termination, and the final report. The gathered
 // vectors are in shared memory where they fit (some 20,000 rows and columns together), the matrix too
-// where it fits beside them, else streamed from L2; larger LPs pass the gathered vector through shared
-// memory in windows. An LP runs for at
-// most `chunk_attempts` attempts per launch and keeps its state in device memory between
-// launches, so a host loop can admit and retire LPs between launches.
+// where it fits beside them, else streamed from L2; of larger LPs the gathered vector alone (up to 27,136
+// entries), and beyond that its entries are gathered out of L2, by clusters in a launch of their own
+// that leaves the shared memory to L1. An LP runs for at most `chunk_attempts` attempts per launch and keeps
+// its state in device memory between launches, so a host loop can admit and retire LPs between launches.
 //
 // An LP's work partition is built for its group size alone, so its row sums follow the same
 // code and summation order whatever else is in the batch: a result is the same alone and in
@@ -23,7 +23,8 @@
 // chain gains more from that than the SM from a second LP. FP64, us per Halpern iteration of one LP alone,
 // gathering from L2 with two blocks a SM before and as here (300 at once, per LP): 2,252 nonzeros 10.2
 // and 3.2 (0.07, 0.03), 15,752: 34 and 13 (0.32, 0.24), 16,561 on a cluster: 15.3 and 4.3 (0.55, 0.32),
-// 112,727: 33 and 17 (2.1, 2.0), 450,562 in windows: 128 and 96.
+// 112,727: 33 and 17 (2.1, 2.0). From L2, alone and of 36 at once: 450,000: 152 and 74 (10.7, 8.1), 1 million
+// (100,000 x 250,000): 367 and 230, 10 million (1,000,000 x 2,500,000): 4,415 and 2,834.
 #pragma once
 
 #include "team_prep.cuh"
@@ -40,7 +41,6 @@ struct BatchSlot {
   RawLp raw;            // what the setup launch prepares the LP from
   const double* start;   // the norm estimate's random start, for S.xc
   const double* x_start;  // the starting point of an LP the host has prepared (raw.v null)
-  int* split;           // a windowed LP's splits: A's, then A's transpose's
   double* zero;         // arrays that start at zero
   size_t zeros;
   double* x_out;    // report: unscaled x, permuted
@@ -82,14 +82,9 @@ __global__ void __launch_bounds__(kThreads) batch_setup_kernel(const NewSlot* fr
     for (int j = base; j < b.P.n; j += stride)
       for (int k = 0; k < 3; ++k) b.raw.x0[k][j] = b.x_start[j];
   team_setup(b.P, b.raw, tm);
-  if (b.plan.windows[0] > 0) {
-    if (tm.cs > 1) tm.sync();
-    else __syncthreads();
-    fill_splits(b.P.A, b.P.m, b.plan.windows[0], b.split, tm);
-    fill_splits(b.P.AT, b.P.n, b.plan.windows[1], b.split + (size_t)(b.plan.windows[0] - 1) * b.P.m, tm);
-  }
 }
 
+template <bool kOnlyL2 = false>
 __device__ __forceinline__ void run_slot(const BatchSlot* from, BatchSlot& b, TeamShared& ts, SideView<double>& sp,
                                          SideView<double>& sd, const Team& tm, long long chunk_attempts) {
   for (int w = threadIdx.x; w < (int)(sizeof(BatchSlot) / 4); w += kThreads)
@@ -103,7 +98,7 @@ __device__ __forceinline__ void run_slot(const BatchSlot* from, BatchSlot& b, Te
     const long long scaled = chunk_attempts * kChunkNnz / per_block;
     chunk_attempts = scaled < 8 ? 8 : scaled;
   }
-  team_solve<double, -1>(b.P, b.S, b.plan, b.plan, b.x_out, b.red_out, b.y_out, ts, sp, sd, sp, sd, b.split, tm,
+  team_solve<double, -1, kOnlyL2>(b.P, b.S, b.plan, b.plan, b.x_out, b.red_out, b.y_out, ts, sp, sd, sp, sd, tm,
                          chunk_attempts, 1 << 30);
 }
 
@@ -127,6 +122,8 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const BatchSlot* slo
   }
 }
 
+// kOnlyL2: for LPs gathered out of L2, launched without dynamic shared memory.
+template <bool kOnlyL2>
 __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kThreads, 1)
     cluster_batch_kernel(const BatchSlot* slots, const int* active, const int* active_count,
                          int* queue_head, long long chunk_attempts) {
@@ -143,7 +140,7 @@ __global__ void __cluster_dims__(kClusterSize, 1, 1) __launch_bounds__(kThreads,
     const int q = *cl.map_shared_rank(&s_take, 0);
     cl.sync();
     if (q >= count) break;
-    run_slot(slots + active[q], b, ts, sp, sd, tm, chunk_attempts);
+    run_slot<kOnlyL2>(slots + active[q], b, ts, sp, sd, tm, chunk_attempts);
   }
 }
 

@@ -7,7 +7,7 @@
 // cluster when the LP has at least cluster_min_nnz nonzeros); step() admits waiting LPs that fit the
 // pool -- one copy each, then one launch in which a block or cluster per LP scales and lays it out
 // (team_prep.cuh) -- replays the graph (the single-block and the cluster
-// persistent kernels side by side on two forked streams, over every active LP of their
+// persistent kernels side by side on forked streams, over every active LP of their
 // class, each LP for at most chunk_attempts attempts),
 // reads the compact control blocks back, re-checks every Farkas certificate on the host, and
 // retires finished LPs with their answers. LPs admitted while others run simply join the
@@ -62,6 +62,12 @@ struct PartOff {
   size_t blk_seg_begin, segs, blk_long_begin, longs, blk_item_begin, items, seg_sum, sell_idx, sell_val;
 };
 
+// The classes of LPs, each with a queue and a launch of its own: a block an LP, a cluster, and a cluster for
+// LPs whose entries are gathered out of L2, which leave the shared memory to L1: in one launch with the others
+// (212 KB a block, some 16 KB of L1) such an LP took 2 to 2.5 times as long an iteration (1 million nonzeros,
+// 100,000 x 250,000, 8 blocks: 497 us, 230 in a launch of its own).
+enum { kOneBlock = 0, kCluster = 1, kClusterL2 = 2, kKinds = 3 };
+
 // One submitted LP.
 struct Job {
   int64_t ticket = 0;
@@ -84,7 +90,7 @@ struct Job {
     PartOff pa, pat;
     size_t c, scl, scu, srl, sru, dr, dc, c0, cl0, cu0, rl0, ru0;
     size_t row_pos, col_pos, next, ecol, ev, rp, cp;
-    size_t split, zero, zeros;
+    size_t zero, zeros;
     size_t x0, x1, y0, y1, ax0, ax1, xsum, ysum, xr, yr, best_x, best_y;
     size_t xt, yt, axr;  // the Halpern operator's T(z) and A x_0
     size_t xc, yc;       // both candidates of an evaluation; then the report's x, reduced costs and y
@@ -93,6 +99,7 @@ struct Job {
   Ctrl ctrl0{};
   // lifecycle
   int group = 1;  // blocks working on this LP: 1, or kClusterSize
+  int kind() const { return group == 1 ? kOneBlock : plan.outside == kFromL2 ? kClusterL2 : kCluster; }
   int slot = -1;
   unsigned char* base = nullptr;  // its device region: in the pool at pool_offset, or
   size_t pool_offset = 0;
@@ -164,7 +171,7 @@ void prepare(Job& J, const sankhya_pdhg_problem& p, const sankhya_pdhg_params& p
     pat = partition(q.at_ptr, J.group, kWarps, prm.group_size_cols, Schedule{}, true);
     J.plan = plan_resident(m, n, q.at_ptr, q.a_ptr, pat, pa, J.group, 8,
                            prm.algorithm == SANKHYA_PDHG_ALGORITHM_HALPERN, true);
-    if (J.plan.cs == 0) J.plan = plan_windows(m, n, J.group);
+    if (J.plan.cs == 0) J.plan = plan_outside(m, n, J.group);
     o.a_ptr = L.put((um + 1) * 4);
     o.at_ptr = L.put((un + 1) * 4);
     o.rptr = L.put((um + 1) * 4);
@@ -221,8 +228,6 @@ void prepare(Job& J, const sankhya_pdhg_problem& p, const sankhya_pdhg_params& p
     o.cp = L.put(un * 16);
     o.xc = L.put(un * 16);
     o.yc = L.put(um * 16);
-    o.split = L.put(4 * (static_cast<size_t>(std::max(0, J.plan.windows[0] - 1)) * um +
-                         static_cast<size_t>(std::max(0, J.plan.windows[1] - 1)) * un));
     o.zero = L.bytes;
     for (size_t* f : {&o.x0, &o.x1, &o.xsum, &o.xr, &o.best_x, &o.ray_out, &o.xt}) *f = L.put(un * 8);
     for (size_t* f : {&o.y0, &o.y1, &o.ax0, &o.ax1, &o.ysum, &o.yr, &o.best_y, &o.farkas_out, &o.yt, &o.axr})
@@ -385,28 +390,30 @@ struct Server {
   BatchSlot* d_slots = nullptr;
   NewSlot* d_fresh = nullptr;  // the LPs being admitted
   Ctrl* d_ctrls = nullptr;
-  Ctrl* d_compact = nullptr;
-  // per class (0: one block per LP, 1: a cluster per LP): active list, count, queue head
-  int* d_active[2] = {nullptr, nullptr};
-  int* d_count[2] = {nullptr, nullptr};
-  int* d_head[2] = {nullptr, nullptr};
-  Ctrl* d_compact2 = nullptr;
-  Ctrl* h_compact = nullptr;
-  Ctrl* h_compact2 = nullptr;
-  int* h_active = nullptr;
-  int* h_active2 = nullptr;
-  int* h_counts = nullptr;
+  struct Class {
+    std::vector<int> active;  // slot indices, largest LP first
+    // on the device: active list, count, queue head, and the active LPs' control blocks
+    int *d_active = nullptr, *d_count = nullptr, *d_head = nullptr;
+    Ctrl* d_compact = nullptr;
+    // pinned mirrors
+    Ctrl* h_compact = nullptr;
+    int *h_active = nullptr, *h_count = nullptr;
+  } cls[kKinds];
+  size_t running() const {
+    size_t n = 0;
+    for (const Class& c : cls) n += c.active.size();
+    return n;
+  }
   cudaGraphExec_t graph = nullptr;
-  // the split of the GPU between the two classes: clusters for the large LPs, single blocks
+  // the split of the GPU between the classes: clusters for the large LPs, single blocks
   // for the others; chosen per round from the active work, the graph rebuilt when it changes
   int slots_total = 0;     // co-resident blocks of the batch kernels
   int max_clusters = 0;    // co-resident 8-block clusters
-  int clusters = 0;        // clusters of the current graph
+  int clusters = 0;        // clusters of the current graph, of both kinds
+  int l2_clusters = 0;     // of them, for the LPs gathered out of L2
   int small_grid = 0;      // single blocks of the current graph
   std::vector<int> free_slots;
   std::vector<std::shared_ptr<Job>> slot_job;
-  std::vector<int> active;  // slot indices, largest LP first
-  std::vector<int> active_big;  // the same for the cluster class
   std::deque<std::shared_ptr<Job>> waiting;
   std::deque<std::shared_ptr<Job>> solo_waiting;  // LPs the single-LP engine solves alone
   std::map<int64_t, std::shared_ptr<Job>> jobs;
@@ -521,7 +528,6 @@ BatchSlot relocate(const Job& J, unsigned char* base, Ctrl* ctrl) {
   R.x0[2] = S.best_x;
   b.start = D(o.start);
   b.x_start = D(o.x_start);
-  b.split = I(o.split);
   b.zero = D(o.zero);
   b.zeros = o.zeros;
   // the report's outputs go where the evaluations kept their candidates
@@ -536,9 +542,12 @@ void query_capacity(Server& s) {
   int bpsm = 0;
   SIH26_SCUDA(cudaFuncSetAttribute(batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kResidentBytes), SANKHYA_GPU_INIT_FAILED);
-  SIH26_SCUDA(cudaFuncSetAttribute(cluster_batch_kernel,
+  SIH26_SCUDA(cudaFuncSetAttribute(cluster_batch_kernel<false>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    kResidentBytes), SANKHYA_GPU_INIT_FAILED);
+  // asked for: an SM otherwise keeps the split of the launch before (a round of such LPs 14.2 ms, 13.0 with it)
+  SIH26_SCUDA(cudaFuncSetAttribute(cluster_batch_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                   (int)cudaSharedmemCarveoutMaxL1), SANKHYA_GPU_INIT_FAILED);
   SIH26_SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, batch_kernel, kThreads,
                                                             kResidentBytes),
               SANKHYA_GPU_INIT_FAILED);
@@ -558,53 +567,66 @@ void query_capacity(Server& s) {
   lc.attrs = &attr;
   lc.numAttrs = 1;
   int max_clusters = 0;
-  SIH26_SCUDA(cudaOccupancyMaxActiveClusters(&max_clusters, cluster_batch_kernel, &lc),
+  SIH26_SCUDA(cudaOccupancyMaxActiveClusters(&max_clusters, cluster_batch_kernel<false>, &lc),
               SANKHYA_GPU_INIT_FAILED);
   // keep at least one cluster's worth of blocks for the single-block class
   s.max_clusters = std::max(1, std::min(max_clusters, (s.slots_total - kClusterSize) / kClusterSize));
 }
 
-// The round's graph for `clusters` 8-block clusters and the remaining blocks as single blocks:
-// the two persistent kernels side by side on two forked streams, then the control blocks of
-// both classes compacted for the host.
-void build_graph(Server& s, int clusters) {
-  clusters = std::max(1, std::min(clusters, s.max_clusters));
-  const int small_grid = std::max(1, s.slots_total - clusters * kClusterSize);
-  if (s.graph && clusters == s.clusters && small_grid == s.small_grid && s.chunk == s.graph_chunk)
+// The round's graph for `clusters` 8-block clusters, as many again as `l2` for the LPs gathered out of L2, and
+// the remaining blocks as single blocks: the persistent kernels side by side on forked streams, then the control
+// blocks of each class compacted for the host. A class of clusters without any has no launch.
+void build_graph(Server& s, int clusters, int l2) {
+  const int small_grid = std::max(1, s.slots_total - (clusters + l2) * kClusterSize);
+  if (s.graph && clusters == s.clusters - s.l2_clusters && l2 == s.l2_clusters && small_grid == s.small_grid &&
+      s.chunk == s.graph_chunk)
     return;
   if (s.graph) {
     cudaGraphExecDestroy(s.graph);
     s.graph = nullptr;
   }
-  cudaStream_t cap, side;
+  cudaStream_t cap, side[kKinds];  // side[0] unused
+  cudaEvent_t fork, join[kKinds];
   SIH26_SCUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking), SANKHYA_GPU_INIT_FAILED);
-  SIH26_SCUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), SANKHYA_GPU_INIT_FAILED);
-  cudaEvent_t fork, join;
   SIH26_SCUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), SANKHYA_GPU_INIT_FAILED);
-  SIH26_SCUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming), SANKHYA_GPU_INIT_FAILED);
+  for (int k = kCluster; k < kKinds; ++k) {
+    SIH26_SCUDA(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking), SANKHYA_GPU_INIT_FAILED);
+    SIH26_SCUDA(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming), SANKHYA_GPU_INIT_FAILED);
+  }
   const long long chunk = s.chunk;
   cudaGraph_t g;
   SIH26_SCUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), SANKHYA_GPU_INIT_FAILED);
-  cudaMemsetAsync(s.d_head[0], 0, sizeof(int), cap);
-  cudaMemsetAsync(s.d_head[1], 0, sizeof(int), cap);
+  for (const Server::Class& c : s.cls) cudaMemsetAsync(c.d_head, 0, sizeof(int), cap);
   cudaEventRecord(fork, cap);
-  cudaStreamWaitEvent(side, fork, 0);
-  cluster_batch_kernel<<<clusters * kClusterSize, kThreads, kResidentBytes, side>>>(
-      s.d_slots, s.d_active[1], s.d_count[1], s.d_head[1], chunk);
-  gather_ctrl_kernel<<<64, 128, 0, side>>>(s.d_ctrls, s.d_active[1], s.d_count[1], s.d_compact2);
-  batch_kernel<<<small_grid, kThreads, kResidentBytes, cap>>>(s.d_slots, s.d_active[0],
-                                                                   s.d_count[0], s.d_head[0], chunk);
-  gather_ctrl_kernel<<<128, 128, 0, cap>>>(s.d_ctrls, s.d_active[0], s.d_count[0], s.d_compact);
-  cudaEventRecord(join, side);
-  cudaStreamWaitEvent(cap, join, 0);
+  const int grids[kKinds] = {small_grid, clusters * kClusterSize, l2 * kClusterSize};
+  for (int k = kCluster; k < kKinds; ++k) {
+    if (grids[k] == 0) continue;
+    const Server::Class& c = s.cls[k];
+    cudaStreamWaitEvent(side[k], fork, 0);
+    if (k == kCluster)
+      cluster_batch_kernel<false><<<grids[k], kThreads, kResidentBytes, side[k]>>>(s.d_slots, c.d_active, c.d_count,
+                                                                                  c.d_head, chunk);
+    else
+      cluster_batch_kernel<true><<<grids[k], kThreads, 0, side[k]>>>(s.d_slots, c.d_active, c.d_count, c.d_head, chunk);
+    gather_ctrl_kernel<<<64, 128, 0, side[k]>>>(s.d_ctrls, c.d_active, c.d_count, c.d_compact);
+    cudaEventRecord(join[k], side[k]);
+  }
+  const Server::Class& one = s.cls[kOneBlock];
+  batch_kernel<<<grids[0], kThreads, kResidentBytes, cap>>>(s.d_slots, one.d_active, one.d_count, one.d_head, chunk);
+  gather_ctrl_kernel<<<128, 128, 0, cap>>>(s.d_ctrls, one.d_active, one.d_count, one.d_compact);
+  for (int k = kCluster; k < kKinds; ++k)
+    if (grids[k] > 0) cudaStreamWaitEvent(cap, join[k], 0);
   SIH26_SCUDA(cudaStreamEndCapture(cap, &g), SANKHYA_GPU_INIT_FAILED);
   SIH26_SCUDA(cudaGraphInstantiate(&s.graph, g, 0), SANKHYA_GPU_INIT_FAILED);
   cudaGraphDestroy(g);
   cudaEventDestroy(fork);
-  cudaEventDestroy(join);
-  cudaStreamDestroy(side);
+  for (int k = kCluster; k < kKinds; ++k) {
+    cudaEventDestroy(join[k]);
+    cudaStreamDestroy(side[k]);
+  }
   cudaStreamDestroy(cap);
-  s.clusters = clusters;
+  s.l2_clusters = l2;
+  s.clusters = clusters + l2;
   s.small_grid = small_grid;
   s.graph_chunk = chunk;
 }
@@ -678,6 +700,22 @@ int clusters_for_round(const Server& s, long long small_nnz, long long big_nnz, 
   want = std::min(want, big_count);
   if (small_nnz > 0) want = std::min(want, s.max_clusters);
   return std::max(1, want);
+}
+
+// Of them, those for the LPs gathered out of L2: as many as there are where every large LP has a cluster, else
+// their share of the large LPs' nonzeros, at least one and one less than all where there are others. Rounded up:
+// an LP that waits for a cluster takes a round twice as long, and these have the longest.
+int l2_clusters_for_round(const Server& s, int clusters, long long big_nnz, long long l2_nnz) {
+  const int count = static_cast<int>(s.cls[kClusterL2].active.size());
+  const int others = static_cast<int>(s.cls[kCluster].active.size());
+  if (count == 0) return 0;
+  if (others == 0) return clusters;
+  if (count + others <= clusters) return count;
+  const double share = static_cast<double>(l2_nnz) / static_cast<double>(std::max(1ll, big_nnz));
+  const int want = std::max(1, std::min({count, clusters - 1, static_cast<int>(std::ceil(share * clusters))}));
+  // hysteresis: a few too many are not worth a new graph
+  const int now = s.l2_clusters;
+  return now >= want && now - want <= now / 4 && now < clusters && now <= count ? now : want;
 }
 
 // Bytes of the report's outputs, from off.xc on.
@@ -754,7 +792,7 @@ void finish_job(Server& s, Job& J, const Ctrl& c, const unsigned char* out) {
 static void solve_one_solo(Server& s);
 
 static void run_solo(Server& s) {
-  const bool batch_idle = s.active.empty() && s.active_big.empty() && s.waiting.empty();
+  const bool batch_idle = s.running() == 0 && s.waiting.empty();
   const double budget = batch_idle ? 1e30 : s.last_round_seconds;
   const double start = s.now();
   for (int k = 0; k < 16 && !s.solo_waiting.empty(); ++k) {
@@ -850,7 +888,7 @@ static void admit(Server& s) {
     f.index = slot;
     fresh[J->group > 1].push_back(f);
     s.slot_job[slot] = J;
-    (J->group > 1 ? s.active_big : s.active).push_back(slot);
+    s.cls[J->kind()].active.push_back(slot);
     note_family(s, *J);
   }
   if (fresh[0].empty() && fresh[1].empty()) return;
@@ -878,8 +916,7 @@ static void admit(Server& s) {
   }
   // the copies above read `fresh`: staged by the runtime, as pageable memory is, before they return
   const auto larger = [&](int a, int b) { return s.slot_job[a]->nnz > s.slot_job[b]->nnz; };
-  std::stable_sort(s.active.begin(), s.active.end(), larger);
-  std::stable_sort(s.active_big.begin(), s.active_big.end(), larger);
+  for (Server::Class& c : s.cls) std::stable_sort(c.active.begin(), c.active.end(), larger);
 }
 
 // Handles the LPs of one class whose control blocks came back in `compact`; returns those
@@ -955,44 +992,40 @@ static std::vector<int> settle(Server& s, const std::vector<int>& list, const Ct
 }
 
 static void run_round(Server& s) {
-  const int c0 = static_cast<int>(s.active.size()), c1 = static_cast<int>(s.active_big.size());
-  if (c0 + c1 == 0) return;
-  long long small_nnz = 0, big_nnz = 0;
-  for (int slot : s.active) small_nnz += s.slot_job[slot]->nnz;
-  for (int slot : s.active_big) big_nnz += s.slot_job[slot]->nnz;
-  int want = clusters_for_round(s, small_nnz, big_nnz, c1);
-  // hysteresis: a small change of the ideal split is not worth a new graph
+  if (s.running() == 0) return;
+  long long nnz[kKinds] = {0, 0, 0};
+  for (int k = 0; k < kKinds; ++k)
+    for (int slot : s.cls[k].active) nnz[k] += s.slot_job[slot]->nnz;
+  const long long big_nnz = nnz[kCluster] + nnz[kClusterL2];
+  int want = clusters_for_round(s, nnz[kOneBlock], big_nnz, static_cast<int>(s.running() - s.cls[kOneBlock].active.size()));
+  // hysteresis, as above
   if (s.graph && std::abs(want - s.clusters) <= std::max(1, s.clusters / 4)) want = s.clusters;
-  build_graph(s, want);
-  std::memcpy(s.h_active, s.active.data(), c0 * sizeof(int));
-  std::memcpy(s.h_active2, s.active_big.data(), c1 * sizeof(int));
-  s.h_counts[0] = c0;
-  s.h_counts[1] = c1;
-  if (c0)
-    SIH26_SCUDA(cudaMemcpyAsync(s.d_active[0], s.h_active, c0 * sizeof(int),
-                                cudaMemcpyHostToDevice, s.stream), SANKHYA_GPU_COPY_FAILED);
-  if (c1)
-    SIH26_SCUDA(cudaMemcpyAsync(s.d_active[1], s.h_active2, c1 * sizeof(int),
-                                cudaMemcpyHostToDevice, s.stream), SANKHYA_GPU_COPY_FAILED);
-  SIH26_SCUDA(cudaMemcpyAsync(s.d_count[0], &s.h_counts[0], sizeof(int), cudaMemcpyHostToDevice,
-                              s.stream), SANKHYA_GPU_COPY_FAILED);
-  SIH26_SCUDA(cudaMemcpyAsync(s.d_count[1], &s.h_counts[1], sizeof(int), cudaMemcpyHostToDevice,
-                              s.stream), SANKHYA_GPU_COPY_FAILED);
+  want = std::max(1, std::min(want, s.max_clusters));
+  const int l2 = l2_clusters_for_round(s, want, big_nnz, nnz[kClusterL2]);
+  // a class with LPs always gets a cluster (one that does not fit beside the others waits for them)
+  build_graph(s, std::max(want - l2, s.cls[kCluster].active.empty() ? 0 : 1), l2);
+  for (Server::Class& c : s.cls) {
+    const size_t count = c.active.size();
+    *c.h_count = static_cast<int>(count);
+    SIH26_SCUDA(cudaMemcpyAsync(c.d_count, c.h_count, sizeof(int), cudaMemcpyHostToDevice, s.stream),
+                SANKHYA_GPU_COPY_FAILED);
+    if (count == 0) continue;
+    std::memcpy(c.h_active, c.active.data(), count * sizeof(int));
+    SIH26_SCUDA(cudaMemcpyAsync(c.d_active, c.h_active, count * sizeof(int), cudaMemcpyHostToDevice, s.stream),
+                SANKHYA_GPU_COPY_FAILED);
+  }
   const double started = s.now();
   SIH26_SCUDA(cudaGraphLaunch(s.graph, s.stream), SANKHYA_GPU_KERNEL_LAUNCH_FAILED);
   ++s.launches;
   ++s.rounds;
-  if (c0)
-    SIH26_SCUDA(cudaMemcpyAsync(s.h_compact, s.d_compact, c0 * sizeof(Ctrl),
-                                cudaMemcpyDeviceToHost, s.stream), SANKHYA_GPU_COPY_FAILED);
-  if (c1)
-    SIH26_SCUDA(cudaMemcpyAsync(s.h_compact2, s.d_compact2, c1 * sizeof(Ctrl),
-                                cudaMemcpyDeviceToHost, s.stream), SANKHYA_GPU_COPY_FAILED);
+  for (Server::Class& c : s.cls)
+    if (!c.active.empty())
+      SIH26_SCUDA(cudaMemcpyAsync(c.h_compact, c.d_compact, c.active.size() * sizeof(Ctrl), cudaMemcpyDeviceToHost,
+                                  s.stream), SANKHYA_GPU_COPY_FAILED);
   SIH26_SCUDA(cudaStreamSynchronize(s.stream), SANKHYA_GPU_SYNC_FAILED);
   s.last_round_seconds = s.now() - started;
   s.round_work = 0.0;
-  s.active = settle(s, s.active, s.h_compact);
-  s.active_big = settle(s, s.active_big, s.h_compact2);
+  for (Server::Class& c : s.cls) c.active = settle(s, c.active, c.h_compact);
   tune_chunk(s);
 }
 
@@ -1060,7 +1093,7 @@ int sankhya_pdhg_server_create(const sankhya_pdhg_server_config* config,
     const size_t ctrls_b = (cap * sizeof(sih26::Ctrl) + 255) & ~size_t(255);
     const size_t list_b = (cap * sizeof(int) + 255) & ~size_t(255);
     const size_t fresh_b = (cap * sizeof(sih26::NewSlot) + 255) & ~size_t(255);
-    s->table_chunk = chunk(slots_b + fresh_b + 3 * ctrls_b + 2 * (list_b + 512) + 256);
+    s->table_chunk = chunk(slots_b + fresh_b + (1 + sih26::kKinds) * ctrls_b + sih26::kKinds * (list_b + 512) + 256);
     unsigned char* at = static_cast<unsigned char*>(s->table_chunk.p);
     const auto carve = [&](size_t bytes) {
       unsigned char* p = at;
@@ -1070,27 +1103,26 @@ int sankhya_pdhg_server_create(const sankhya_pdhg_server_config* config,
     s->d_slots = reinterpret_cast<sih26::BatchSlot*>(carve(slots_b));
     s->d_fresh = reinterpret_cast<sih26::NewSlot*>(carve(fresh_b));
     s->d_ctrls = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
-    s->d_compact = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
-    s->d_compact2 = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
-    for (int k = 0; k < 2; ++k) {
-      s->d_active[k] = reinterpret_cast<int*>(carve(list_b));
-      s->d_count[k] = reinterpret_cast<int*>(carve(256));
-      s->d_head[k] = reinterpret_cast<int*>(carve(256));
-      SIH26_SCUDA(cudaMemsetAsync(s->d_count[k], 0, sizeof(int), s->stream), SANKHYA_GPU_INIT_FAILED);
+    for (Server::Class& c : s->cls) {
+      c.d_compact = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
+      c.d_active = reinterpret_cast<int*>(carve(list_b));
+      c.d_count = reinterpret_cast<int*>(carve(256));
+      c.d_head = reinterpret_cast<int*>(carve(256));
+      SIH26_SCUDA(cudaMemsetAsync(c.d_count, 0, sizeof(int), s->stream), SANKHYA_GPU_INIT_FAILED);
     }
     unsigned long long* d_clock = reinterpret_cast<unsigned long long*>(carve(256));
-    s->pinned_chunk = cache.take_pinned(2 * ctrls_b + 2 * list_b + 256);
+    s->pinned_chunk = cache.take_pinned(sih26::kKinds * (ctrls_b + list_b + 256));
     if (!s->pinned_chunk) throw Failure{SANKHYA_GPU_OUT_OF_MEMORY, "cudaMallocHost: out of memory"};
     at = static_cast<unsigned char*>(s->pinned_chunk.p);
-    s->h_compact = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
-    s->h_compact2 = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
-    s->h_active = reinterpret_cast<int*>(carve(list_b));
-    s->h_active2 = reinterpret_cast<int*>(carve(list_b));
-    s->h_counts = reinterpret_cast<int*>(carve(256));
+    for (Server::Class& c : s->cls) {
+      c.h_compact = reinterpret_cast<sih26::Ctrl*>(carve(ctrls_b));
+      c.h_active = reinterpret_cast<int*>(carve(list_b));
+      c.h_count = reinterpret_cast<int*>(carve(256));
+    }
     s->slot_job.resize(cap);
     for (int k = cap - 1; k >= 0; --k) s->free_slots.push_back(k);
     sih26::query_capacity(*s);
-    sih26::build_graph(*s, s->cfg.clusters > 0 ? s->cfg.clusters : 16);
+    sih26::build_graph(*s, std::min(s->cfg.clusters > 0 ? s->cfg.clusters : 16, s->max_clusters), 0);
     sih26::read_clock<<<1, 1, 0, s->stream>>>(d_clock);
     SIH26_SCUDA(cudaMemcpyAsync(&s->device_clock0, d_clock, sizeof *d_clock,
                                 cudaMemcpyDeviceToHost, s->stream), SANKHYA_GPU_COPY_FAILED);
@@ -1188,7 +1220,7 @@ int sankhya_pdhg_server_step(sankhya_pdhg_server* server, int32_t* active, int32
     sih26::g_last_error = f.message;
     return f.code;
   }
-  if (active) *active = static_cast<int32_t>(s->active.size() + s->active_big.size());
+  if (active) *active = static_cast<int32_t>(s->running());
   if (waiting) *waiting = static_cast<int32_t>(s->waiting.size() + s->solo_waiting.size());
   if (finished) {
     int32_t k = 0;

@@ -816,43 +816,18 @@ __device__ __noinline__ void team_attempt(const ResidentPlan& pl,
   finish_attempt(ts, tm, acc);
 }
 
-// ---- an LP whose vectors do not fit: the gathered vector in windows -------------------------------
+// ---- an LP whose vectors do not fit beside each other -------------------------------------------------
 //
 // s_r = sum_k val vec[idx] over this block's rows, then the epilogue (the grid-wide kernels', whose
-// inputs are in global memory). The block reads the vector window by window into shared memory,
-// coalesced, and passes over its rows once per window: a row's entries are in ascending order, so
-// those of a window are the range between two splits (found once per LP), and its sum so far waits
-// in `partial` between windows. Bound by reading the matrix and the vector from L2 (12 bytes an
-// entry and 8 bytes per column and row and block); gathering the vector's entries from L2 instead moves a
-// 32-byte sector for each: 450,000 nonzeros on 8 blocks took 153 us an iteration that way.
-struct Windows {
-  int count;
-  int rows;          // of the matrix: stride of splits
-  const int* split;  // [count - 1][rows]: entries of row r in windows 0 .. w
-  double* partial;   // [rows], stride 2 doubles (a candidate pair's array, free between evaluations)
-};
-
-// Splits of this block's rows (every kind), by binary search.
-__device__ inline void fill_splits(const Csr<double>& M, int rows, int count, int* split, const Team& tm) {
-  for (int w = 0; w + 1 < count; ++w)
-    for (int r = tm.rank * kThreads + threadIdx.x; r < rows; r += tm.cs * kThreads) {
-      const int b = M.ptr[r], e = M.ptr[r + 1], limit = (w + 1) * kWindow;
-      int lo = b, hi = e;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (M.idx[mid] < limit) lo = mid + 1;
-        else hi = mid;
-      }
-      split[(size_t)w * rows + r] = lo - b;
-    }
-}
-
+// inputs are in global memory). The block copies the gathered vector into shared memory, coalesced, and
+// passes over its rows. Bound by reading the matrix and the vector from L2 (12 bytes an entry and
+// 8 bytes per column and row and block); gathering the vector's entries from L2 instead moves a 32-byte
+// sector for each that L1 does not hold.
 template <int NS, bool kRound, class Epi>
-__device__ __forceinline__ void window_phase(const Csr<double>& M, const Part& p, const Windows& win,
-                                             const double* vec, int size, double scale, const Epi& epi,
-                                             double (&acc)[NS], int rank) {
+__device__ __forceinline__ void turn_phase(const Csr<double>& M, const Part& p, const double* vec, int size,
+                                           double scale, const Epi& epi, double (&acc)[NS], int rank) {
   constexpr int U = 8;
-  double* const mem = reinterpret_cast<double*>(team_memory());
+  double* const g = reinterpret_cast<double*>(team_memory());
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ib = __ldg(p.blk_item_begin + rank), ie = __ldg(p.blk_item_begin + rank + 1);
   const int lb = __ldg(p.blk_long_begin + rank), le = __ldg(p.blk_long_begin + rank + 1);
@@ -862,151 +837,129 @@ __device__ __forceinline__ void window_phase(const Csr<double>& M, const Part& p
     if constexpr (kRound) return __dadd_rn(s, __dmul_rn(a, x));
     else return s + a * x;
   };
-  for (int w = 0; w < win.count; ++w) {
-    const int from = w * kWindow, entries = size - from < kWindow ? size - from : kWindow;
-    const bool first = w == 0, last = w + 1 == win.count;
-    __syncthreads();  // the window before is done with
-    {
-      // vectors start on 256 bytes and windows on 16: two entries a load
-      const double2* src = reinterpret_cast<const double2*>(vec + from);
-      double2* dst = reinterpret_cast<double2*>(mem);
+  __syncthreads();  // the vector before is done with
+  {
+    // vectors start on 256 bytes: two entries a load
+    const double2* src = reinterpret_cast<const double2*>(vec);
+    double2* dst = reinterpret_cast<double2*>(g);
 #pragma unroll 8
-      for (int k = threadIdx.x; k < entries / 2; k += kThreads) {
-        double2 t = src[k];
-        if constexpr (kRound) {
-          t.x *= scale;
-          t.y *= scale;
-        }
-        dst[k] = t;
+    for (int k = threadIdx.x; k < size / 2; k += kThreads) {
+      double2 t = src[k];
+      if constexpr (kRound) {
+        t.x *= scale;
+        t.y *= scale;
       }
-      if ((entries & 1) && threadIdx.x == 0)
-        mem[entries - 1] = kRound ? vec[from + entries - 1] * scale : vec[from + entries - 1];
+      dst[k] = t;
     }
-    __syncthreads();
-    const double* const g = mem - from;
-    const auto begin_of = [&](int r) { return first ? 0 : __ldg(win.split + (size_t)(w - 1) * win.rows + r); };
-    const auto end_of = [&](int r, int len) { return last ? len : __ldg(win.split + (size_t)w * win.rows + r); };
-    for (int q = lb + warp; q < le; q += kWarps) {  // long rows: a warp each
-      const int r = __ldg(p.longs + q).x, b = __ldg(M.ptr + r), len = __ldg(M.ptr + r + 1) - b;
-      typename Epi::In in{};
-      if (last && lane == 0) in = epi.load(r);
-      const int k1 = end_of(r, len);
-      double s[1] = {0.0};
+    if ((size & 1) && threadIdx.x == 0) g[size - 1] = kRound ? vec[size - 1] * scale : vec[size - 1];
+  }
+  __syncthreads();
+  for (int q = lb + warp; q < le; q += kWarps) {  // long rows: a warp each
+    const int r = __ldg(p.longs + q).x, b = __ldg(M.ptr + r), e = __ldg(M.ptr + r + 1);
+    typename Epi::In in{};
+    if (lane == 0) in = epi.load(r);
+    double s[1] = {0.0};
 #pragma unroll 4
-      for (int k = begin_of(r) + lane; k < k1; k += 32) s[0] += __ldg(M.val64 + b + k) * g[__ldg(M.idx + b + k)];
+    for (int k = b + lane; k < e; k += 32) s[0] += __ldg(M.val64 + k) * g[__ldg(M.idx + k)];
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
-      if (lane == 0) {
-        if (!first) s[0] += win.partial[2 * (size_t)r];
-        if (last) epi.apply(r, s, in, acc);
-        else win.partial[2 * (size_t)r] = s[0];
-      }
+    for (int off = 16; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
+    if (lane == 0) epi.apply(r, s, in, acc);
+  }
+  // the headers of the warp's next rows are on their way while these are summed: the item two
+  // ahead, its rows' range one ahead
+  struct Header {
+    int b, len;
+  };
+  const auto lane_row = [&](const int4& item) { return item.z < 0 ? item.x + lane : item.x + lane / item.z; };
+  const auto header = [&](const int4& item) {
+    Header h{0, 0};
+    const int r = lane_row(item);
+    if (r < item.y) {
+      h.b = __ldg(M.ptr + r);
+      h.len = __ldg(M.ptr + r + 1) - h.b;
     }
-    // the headers of the warp's next rows are on their way while these are summed: the item two
-    // ahead, its rows' range one ahead
-    struct Header {
-      int b, k0, k1;
-      double sum;
-    };
-    const auto lane_row = [&](const int4& item) {
-      return item.z < 0 ? item.x + lane : item.x + lane / item.z;
-    };
-    const auto header = [&](const int4& item) {
-      Header h{0, 0, 0, 0.0};
-      const int r = lane_row(item);
-      if (r < item.y) {
-        h.b = __ldg(M.ptr + r);
-        const int len = __ldg(M.ptr + r + 1) - h.b;
-        h.k0 = begin_of(r);
-        h.k1 = end_of(r, len);
-        if (!first) h.sum = win.partial[2 * (size_t)r];
+    return h;
+  };
+  const int4 none = make_int4(0, 0, -1, 0);
+  int it = ib + warp;
+  int4 item = it < ie ? __ldg(p.items + it) : none;
+  int4 next = it + kWarps < ie ? __ldg(p.items + it + kWarps) : none;
+  Header h = header(item);
+  for (; it < ie; it += kWarps) {
+    const int4 after = it + 2 * kWarps < ie ? __ldg(p.items + it + 2 * kWarps) : none;
+    const Header hn = header(next);
+    const int rows = item.y - item.x, r = lane_row(item);
+    const bool mine = r < item.y;
+    typename Epi::In in{};
+    double s[1] = {0.0};
+    if (item.z < 0) {
+      if (mine) in = epi.load(r);
+      const int* si = sidx + item.w + lane;
+      const double* sv = sval + item.w + lane;
+      for (int k = 0; __any_sync(0xffffffffu, k < h.len); k += U) {
+        int j[U];
+        double a[U];
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+          const bool live = k + t < h.len;
+          j[t] = live ? __ldg(si + (k + t) * rows) : 0;
+          a[t] = live ? __ldg(sv + (k + t) * rows) : 0.0;
+        }
+#pragma unroll
+        for (int t = 0; t < U; ++t)
+          if (k + t < h.len) s[0] = add(s[0], a[t], g[j[t]]);
       }
-      return h;
-    };
-    const int4 none = make_int4(0, 0, -1, 0);
-    int it = ib + warp;
-    int4 item = it < ie ? __ldg(p.items + it) : none;
-    int4 next = it + kWarps < ie ? __ldg(p.items + it + kWarps) : none;
-    Header h = header(item);
-    for (; it < ie; it += kWarps) {
-      const int4 after = it + 2 * kWarps < ie ? __ldg(p.items + it + 2 * kWarps) : none;
-      const Header hn = header(next);
-      const int rows = item.y - item.x, r = lane_row(item);
-      const bool mine = r < item.y;
-      typename Epi::In in{};
-      double s[1] = {0.0};
-      if (item.z < 0) {
-        if (mine && last) in = epi.load(r);
-        s[0] = h.sum;
-        const int* si = sidx + item.w + lane;
-        const double* sv = sval + item.w + lane;
-        for (int k = h.k0; __any_sync(0xffffffffu, k < h.k1); k += U) {
-          int j[U];
-          double a[U];
-#pragma unroll
-          for (int t = 0; t < U; ++t) {
-            const bool live = k + t < h.k1;
-            j[t] = live ? __ldg(si + (k + t) * rows) : from;
-            a[t] = live ? __ldg(sv + (k + t) * rows) : 0.0;
-          }
-#pragma unroll
-          for (int t = 0; t < U; ++t)
-            if (k + t < h.k1) s[0] = add(s[0], a[t], g[j[t]]);
-        }
-        if (mine) {
-          if (last) epi.apply(r, s, in, acc);
-          else win.partial[2 * (size_t)r] = s[0];
-        }
-      } else {
-        const int lanes = item.z, gl = lane & (lanes - 1);
-        if (mine) {
-          if (last && gl == 0) in = epi.load(r);
+      if (mine) epi.apply(r, s, in, acc);
+    } else {
+      const int lanes = item.z, gl = lane & (lanes - 1);
+      if (mine) {
+        if (gl == 0) in = epi.load(r);
 #pragma unroll 8
-          for (int k = h.k0 + gl; k < h.k1; k += lanes)
-            s[0] += __ldg(M.val64 + h.b + k) * g[__ldg(M.idx + h.b + k)];
-        }
-        for (int off = lanes >> 1; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
-        if (mine && gl == 0) {
-          if (!first) s[0] += h.sum;
-          if (last) epi.apply(r, s, in, acc);
-          else win.partial[2 * (size_t)r] = s[0];
-        }
+        for (int k = gl; k < h.len; k += lanes) s[0] += __ldg(M.val64 + h.b + k) * g[__ldg(M.idx + h.b + k)];
       }
-      item = next;
-      next = after;
-      h = hn;
+      for (int off = lanes >> 1; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
+      if (mine && gl == 0) epi.apply(r, s, in, acc);
     }
+    item = next;
+    next = after;
+    h = hn;
   }
 }
 
-// x's and y's windows of an LP
-__device__ __forceinline__ Windows windows_of(const Prob<double>& P, const State<double>& S, const ResidentPlan& pl,
-                                              const int* split, bool over_x) {
-  // rows of A gather x; rows of A' gather y and their splits follow A's
-  return over_x ? Windows{pl.windows[0], P.m, split, reinterpret_cast<double*>(S.yc)}
-                : Windows{pl.windows[1], P.n, split + (size_t)(pl.windows[0] - 1) * P.m,
-                          reinterpret_cast<double*>(S.xc)};
+// One pass over the rows of a matrix, kTurns: the vector copied into shared memory, else its entries gathered out
+// of L2 by the grid-wide kernels' code.
+template <bool kTurns, int NS, bool kRound, class Epi>
+__device__ __forceinline__ void vector_phase(const Csr<double>& M, const Part& p, const double* vec, int size,
+                                             double scale, const Epi& epi, double (&acc)[NS], int rank) {
+  if constexpr (kTurns) {
+    turn_phase<NS, kRound>(M, p, vec, size, scale, epi, acc, rank);
+  } else if constexpr (kRound) {
+    run_phase<1, NS, false, true, kSliceUnroll, false, true>(M.ptr, M.idx, M.val64, p, ScaledGather{vec, scale}, epi,
+                                                             acc, nullptr, rank);
+  } else {
+    run_phase<1, NS, false, true>(M.ptr, M.idx, M.val64, p, Gather1<double>{vec}, epi, acc, nullptr, rank);
+  }
 }
 
-static __device__ __noinline__ void window_halpern(const Prob<double>& P, const State<double>& S, const ResidentPlan& pl,
-                                            const int* split, TeamShared& ts, const Team& tm_, int steps) {
+template <bool kTurns>
+__device__ __noinline__ void vector_halpern(const Prob<double>& P, const State<double>& S, TeamShared& ts,
+                                            const Team& tm_, int steps) {
   const Team tm = tm_;
   Ctrl& c = ts.c;
-  const Windows wx = windows_of(P, S, pl, split, true), wy = windows_of(P, S, pl, split, false);
   const double tau = c.eta / c.omega, sigma = c.eta * c.omega;
   long long k = c.averaged;
   int cur = c.cur;
   double acc[3] = {0.0, 0.0, 0.0};
   for (int t = 0; t < steps; ++t, ++k, cur ^= 1) {
     const double w = (double)(k + 1) / (double)(k + 2);
-    window_phase<3, false>(P.AT, P.pate, wy, S.y[cur], P.m, 1.0,
-                           PrimalStepHalpern<double>{S.x[cur], S.x[cur ^ 1], S.xt, P.c, P.cl, P.cu, S.xr, tau, w},
-                           acc, tm.rank);
+    vector_phase<kTurns, 3, false>(
+        P.AT, P.pate, S.y[cur], P.m, 1.0,
+        PrimalStepHalpern<double>{S.x[cur], S.x[cur ^ 1], S.xt, P.c, P.cl, P.cu, S.xr, tau, w}, acc, tm.rank);
     tm.sync();
-    window_phase<3, false>(P.A, P.pae, wx, S.x[cur ^ 1], P.n, 1.0,
-                           DualStepHalpern<double>{S.y[cur], S.y[cur ^ 1], S.yt, S.ax[cur ^ 1], P.rl, P.ru, S.yr,
-                                                   S.axr, sigma, w},
-                           acc, tm.rank);
+    vector_phase<kTurns, 3, false>(P.A, P.pae, S.x[cur ^ 1], P.n, 1.0,
+                                   DualStepHalpern<double>{S.y[cur], S.y[cur ^ 1], S.yt, S.ax[cur ^ 1], P.rl, P.ru,
+                                                           S.yr, S.axr, sigma, w},
+                                   acc, tm.rank);
     tm.sync();
   }
   if (threadIdx.x == 0) {
@@ -1020,33 +973,32 @@ static __device__ __noinline__ void window_halpern(const Prob<double>& P, const 
   __syncthreads();
 }
 
-static __device__ __noinline__ void window_attempt(const Prob<double>& P, const State<double>& S, const ResidentPlan& pl,
-                                            const int* split, TeamShared& ts, const Team& tm_) {
+template <bool kTurns>
+__device__ __noinline__ void vector_attempt(const Prob<double>& P, const State<double>& S, TeamShared& ts,
+                                            const Team& tm_) {
   const Team tm = tm_;
   Ctrl& c = ts.c;
-  const Windows wx = windows_of(P, S, pl, split, true), wy = windows_of(P, S, pl, split, false);
   const int cur = c.cur, nxt = cur ^ 1;
   const double tau = c.eta / c.omega, sigma = c.eta * c.omega;
   double acc[3] = {0.0, 0.0, 0.0};
-  window_phase<3, false>(P.AT, P.pate, wy, S.y[cur], P.m, 1.0,
-                         PrimalStep<double>{S.x[cur], S.x[nxt], P.c, P.cl, P.cu, S.xsum, tau, c.pending}, acc,
-                         tm.rank);
+  vector_phase<kTurns, 3, false>(P.AT, P.pate, S.y[cur], P.m, 1.0,
+                                 PrimalStep<double>{S.x[cur], S.x[nxt], P.c, P.cl, P.cu, S.xsum, tau, c.pending},
+                                 acc, tm.rank);
   if (threadIdx.x == kThreads - 1) step_growth(c.iteration, ts.growth[0], ts.growth[1]);
   tm.sync();
-  window_phase<3, false>(P.A, P.pae, wx, S.x[nxt], P.n, 1.0,
-                         DualStep<double>{S.y[cur], S.y[nxt], S.ax[cur], S.ax[nxt], P.rl, P.ru, S.ysum, sigma,
-                                          c.pending},
-                         acc, tm.rank);
+  vector_phase<kTurns, 3, false>(P.A, P.pae, S.x[nxt], P.n, 1.0,
+                                 DualStep<double>{S.y[cur], S.y[nxt], S.ax[cur], S.ax[nxt], P.rl, P.ru, S.ysum,
+                                                  sigma, c.pending},
+                                 acc, tm.rank);
   finish_attempt(ts, tm, acc);
 }
 
-// The norm estimate (team_power) and A x_0 of such an LP. v sits in S.xt while the estimate runs (the
-// candidates' arrays hold the partial sums) and u in S.yt; neither is read before the first step
-// writes it.
-static __device__ __noinline__ double window_setup(const Prob<double>& P, const State<double>& S, const ResidentPlan& pl,
-                                            const int* split, int nnz, TeamShared& ts, const Team& tm_) {
+// The norm estimate (team_power) and A x_0 of such an LP. v sits in S.xt while the estimate runs and u in
+// S.yt; neither is read before the first step writes it.
+template <bool kTurns>
+__device__ __noinline__ double vector_setup(const Prob<double>& P, const State<double>& S, int nnz, TeamShared& ts,
+                                            const Team& tm_) {
   const Team tm = tm_;
-  const Windows wx = windows_of(P, S, pl, split, true), wy = windows_of(P, S, pl, split, false);
   double norm = 1.0;
   if (P.m > 0 && P.n > 0 && nnz > 0) {
     double *v = S.xt, *u = S.yt;
@@ -1066,10 +1018,10 @@ static __device__ __noinline__ double window_setup(const Prob<double>& P, const 
         break;
       }
       double dummy[1] = {0.0};
-      window_phase<1, true>(P.A, P.pae, wx, v, P.n, 1.0 / length, StoreRow<1>{u, -1}, dummy, tm.rank);
+      vector_phase<kTurns, 1, true>(P.A, P.pae, v, P.n, 1.0 / length, StoreRow<1>{u, -1}, dummy, tm.rank);
       tm.sync();
       double nx[1] = {0.0};
-      window_phase<1, true>(P.AT, P.pate, wy, u, P.m, 1.0, StoreRow<1>{v, 0}, nx, tm.rank);
+      vector_phase<kTurns, 1, true>(P.AT, P.pate, u, P.m, 1.0, StoreRow<1>{v, 0}, nx, tm.rank);
       team_part<1, 0u>(ts, 0, nx);
       team_total(ts, tm, 1, 0u);
     }
@@ -1079,7 +1031,7 @@ static __device__ __noinline__ double window_setup(const Prob<double>& P, const 
   }
   double dummy[1] = {0.0};
   const int cur = ts.c.cur;
-  window_phase<1, false>(P.A, P.pae, wx, S.x[cur], P.n, 1.0, StoreRow<1>{S.ax[cur], -1}, dummy, tm.rank);
+  vector_phase<kTurns, 1, false>(P.A, P.pae, S.x[cur], P.n, 1.0, StoreRow<1>{S.ax[cur], -1}, dummy, tm.rank);
   tm.sync();
   for (int i = tm.rank * kThreads + threadIdx.x; i < P.m; i += tm.cs * kThreads) S.axr[i] = S.ax[cur][i];
   return norm;
@@ -1418,29 +1370,33 @@ __device__ __noinline__ void team_report(const Prob<T>& P, const State<T>& S, do
 
 // Runs the LP from its stored state: to a final state, `max_evaluations` evaluations or
 // `max_attempts` attempts, whichever comes first. A final state comes with its report. kHalpern:
-// 1 / 0 for an LP of that operator alone, -1 for either (the batched engine).
-template <class T, int kHalpern>
+// 1 / 0 for an LP of that operator alone, -1 for either (the batched engine). kOnlyL2: for LPs gathered out of
+// L2 alone.
+template <class T, int kHalpern, bool kOnlyL2 = false>
 __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, const ResidentPlan& pl,
                                            const ResidentPlan& pl64, double* x_out, double* red_out, double* y_out,
                                            TeamShared& ts, SideView<T>& sp, SideView<T>& sd, SideView<double>& sp64,
-                                           SideView<double>& sd64, const int* split, const Team& tm,
+                                           SideView<double>& sd64, const Team& tm,
                                            long long max_attempts, int max_evaluations) {
   Ctrl& c = ts.c;
   if (threadIdx.x == 0) c = *S.ctrl;
   tm.sync();  // every block has started: its shared memory may be written
   SIH26_TEAM_MARK(-1);
   const bool halpern = kHalpern >= 0 ? kHalpern != 0 : c.halpern != 0;
-  const bool windowed = kHalpern < 0 && pl.windows[0] > 0;
+  const bool outside = kOnlyL2 || (kHalpern < 0 && pl.outside != kInside);
+  const bool turns = !kOnlyL2 && outside && pl.outside == kInTurns;
   if (c.state == kSetup) {
     SIH26_TEAM_MARK(7);
-    if (pl64.cs > 0 && !windowed) {
+    if (pl64.cs > 0 && !outside) {
       load_side(sp64, pl64.side[0], Csr<double>{P.AT.ptr, P.AT.idx, P.AT.val64, P.AT.val64}, P.pate, P.pate, tm.rank);
       load_side(sd64, pl64.side[1], Csr<double>{P.A.ptr, P.A.idx, P.A.val64, P.A.val64}, P.pae, P.pae, tm.rank);
     }
     double norm;
     const int nnz = __ldg(P.A.ptr + P.m);
     if constexpr (kHalpern < 0) {
-      norm = windowed ? window_setup(P, S, pl, split, nnz, ts, tm) : team_power(P, S, nnz, pl64, sp64, sd64, ts, tm);
+      norm = turns     ? vector_setup<true>(P, S, nnz, ts, tm)
+             : outside ? vector_setup<false>(P, S, nnz, ts, tm)
+                       : team_power(P, S, nnz, pl64, sp64, sd64, ts, tm);
     } else {
       norm = team_power(P, S, nnz, pl64, sp64, sd64, ts, tm);
     }
@@ -1455,8 +1411,8 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
     tm.sync();
   }
   SIH26_TEAM_MARK(9);
-  const bool resident = !windowed;
-  if (windowed && c.state == kSetup) {
+  const bool resident = !outside;
+  if (outside && c.state == kSetup) {
     __syncthreads();
     if (threadIdx.x == 0) c.state = kRunning;
     tm.sync();
@@ -1501,7 +1457,10 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
       if (resident) {
         team_halpern(S, pl, sp, sd, ts, tm, static_cast<int>(steps));
       } else {
-        if constexpr (kHalpern < 0) window_halpern(P, S, pl, split, ts, tm, static_cast<int>(steps));
+        if constexpr (kHalpern < 0) {
+          if (turns) vector_halpern<true>(P, S, ts, tm, static_cast<int>(steps));
+          else vector_halpern<false>(P, S, ts, tm, static_cast<int>(steps));
+        }
       }
       left -= steps;
     } else {
@@ -1509,7 +1468,10 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
         if (resident) {
           team_attempt(pl, sp, sd, ts, tm);
         } else {
-          if constexpr (kHalpern < 0) window_attempt(P, S, pl, split, ts, tm);
+          if constexpr (kHalpern < 0) {
+            if (turns) vector_attempt<true>(P, S, ts, tm);
+            else vector_attempt<false>(P, S, ts, tm);
+          }
         }
         --left;
       } while (c.state == kRunning && left > 0 && c.iteration < c.iteration_limit);
@@ -1557,7 +1519,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     sd64 = &sd;
   }
   const Team tm{pl.cs, pl.cs > 1 ? (int)cooperative_groups::this_cluster().block_rank() : 0};
-  team_solve<T, kHalpern ? 1 : 0>(P, S, pl, pl64, x_out, red_out, y_out, ts, sp, sd, *sp64, *sd64, nullptr, tm,
+  team_solve<T, kHalpern ? 1 : 0>(P, S, pl, pl64, x_out, red_out, y_out, ts, sp, sd, *sp64, *sd64, tm,
                                   max_attempts, max_evaluations);
 }
 

@@ -11,7 +11,7 @@ namespace sih26 {
 
 constexpr int kMaxTeam = 16;                  // blocks of the largest cluster
 constexpr int kResidentBytes = 212 * 1024;    // dynamic shared memory a plan may take (the kernels hold 12 KB more)
-constexpr int kWindow = kResidentBytes / 8;   // FP64 entries of a window
+constexpr int kWholeVector = kResidentBytes / 8;  // FP64 entries of a vector that fits alone
 
 // Where everything sits in a block's dynamic shared memory (bytes; the same in every block of
 // the cluster, sized for the block with the most of each). side[0]: rows of A' (phase P),
@@ -19,9 +19,7 @@ constexpr int kWindow = kResidentBytes / 8;   // FP64 entries of a window
 struct ResidentPlan {
   int cs;      // blocks of the cluster; 0: the LP has no plan
   int bytes;
-  // an LP whose vectors do not fit beside each other: the gathered vector passes through shared memory
-  // in windows of kWindow entries (window_phase); the number of windows of x and y, else 0
-  int windows[2];
+  int outside;         // how an LP whose vectors do not fit beside each other is solved: below
   int x[2], y[2];      // equal: one buffer (the Halpern operator always accepts its step)
   struct Side {
     int resident;      // the entries are in shared memory too
@@ -106,15 +104,23 @@ inline ResidentPlan plan_resident(int m, int n, const std::vector<int>& at_ptr, 
   return pl;
 }
 
-// The same for an LP that has no such plan: windows of x and y, at least one of each: the
-// pass over a side is what applies its rows' steps, also where an LP without rows (or columns) leaves them
-// nothing to gather.
-inline ResidentPlan plan_windows(int m, int n, int cs) {
+// An LP whose vectors do not fit beside each other keeps its state in global memory.
+enum {
+  kInside = 0,
+  kInTurns = 1,  // the gathered vector is copied into shared memory, x and y in turn (turn_phase)
+  kFromL2 = 2    // its entries are gathered out of L2, in a launch without dynamic shared memory
+};
+
+// The plan of such an LP: in turns while either vector fits alone. FP64, us per Halpern iteration of one LP on
+// 8 blocks, and of each of 36 at once, in turns and from L2: 9,000 x 20,000 with 160,000 nonzeros 27 and 18-25,
+// 2.3 and 3.8. Longer vectors in pieces that fit were measured too, and lose: 20,000 x 50,000 with 450,000
+// nonzeros in two pieces 83 and 74 from L2, 11.8 and 8.1 at once; 100,000 x 250,000 with 2.5 million in ten 1,051
+// and 519, 136 and 50; 1,000,000 x 2,500,000 with 10 million in 93 alone 64,831 and 2,834.
+inline ResidentPlan plan_outside(int m, int n, int cs) {
   ResidentPlan pl{};
   pl.cs = cs;
-  pl.bytes = kResidentBytes;
-  pl.windows[0] = n > 0 ? (n + kWindow - 1) / kWindow : 1;
-  pl.windows[1] = m > 0 ? (m + kWindow - 1) / kWindow : 1;
+  pl.outside = std::max(m, n) <= kWholeVector ? kInTurns : kFromL2;
+  pl.bytes = pl.outside == kInTurns ? kResidentBytes : 0;
   return pl;
 }
 
