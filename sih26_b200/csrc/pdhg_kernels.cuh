@@ -1223,7 +1223,10 @@ __global__ void __launch_bounds__(kThreads, 2) iterate_kernel(Prob<T> P, State<T
       run_phase<1, 3, kHalpern, true>(P.A.ptr, P.A.idx, P.A.val, P.pai, gather, step, acc, nullptr);
     }
   };
-  // the step size's growth factors (two pow, 0.8 us), formed at the attempt's first barrier
+  // the step size's growth factors (two pow, 0.8 us): formed at the attempt's first barrier, but not in the plain
+  // FP32 kernel, whose registers that costs more (5M nonzeros, us an attempt: 64.3 and, formed with the step
+  // control, 60.4; FP64 66.0 and 67.9)
+  constexpr bool kEarlyGrowth = kPacked || sizeof(T) == 8;
   __shared__ double growth[2];
   const int G = gridDim.x;
   long long a = 0;
@@ -1282,9 +1285,13 @@ __global__ void __launch_bounds__(kThreads, 2) iterate_kernel(Prob<T> P, State<T
       phase(0, Gather1<T>{S.y[cur]}, ps, acc);
     }
     SIH26_MARK(0);
-    if (!grid_barrier(S.bar, [&] {
-          if (threadIdx.x == kThreads - 1) step_growth(c.iteration, growth[0], growth[1]);
-        })) goto device_error;
+    if constexpr (kEarlyGrowth) {
+      if (!grid_barrier(S.bar, [&] {
+            if (threadIdx.x == kThreads - 1) step_growth(c.iteration, growth[0], growth[1]);
+          })) goto device_error;
+    } else {
+      if (!grid_barrier(S.bar)) goto device_error;
+    }
     SIH26_MARK(1);
 
     if constexpr (kDelta<T>) {
@@ -1304,7 +1311,15 @@ __global__ void __launch_bounds__(kThreads, 2) iterate_kernel(Prob<T> P, State<T
     {
       double tot[3];
       reduce_partials<3, 0u>(part, 0, tot, sh);
-      if (threadIdx.x == 0) step_control(c, tot, growth[0], growth[1]);
+      if (threadIdx.x == 0) {
+        if constexpr (kEarlyGrowth) {
+          step_control(c, tot, growth[0], growth[1]);
+        } else {
+          double shrink, grow;
+          step_growth(c.iteration, shrink, grow);
+          step_control(c, tot, shrink, grow);
+        }
+      }
       __syncthreads();
       SIH26_MARK(4);
       if (c.state != kRunning) break;
