@@ -284,7 +284,11 @@ typedef struct sankhya_pdhg_server sankhya_pdhg_server;
 typedef struct sankhya_pdhg_server_config {
   int32_t device;          /* CUDA device ordinal */
   double memory_fraction;  /* share of free device memory for the pool (default 0.8) */
-  int64_t pool_bytes;      /* explicit pool size; 0 = use memory_fraction */
+  int64_t pool_bytes;      /* explicit pool size; 0 = use memory_fraction. An LP takes about 49
+                              bytes per nonzero and up to 300 per row and column of it while it
+                              runs. One that needs more than the pool, but whose two matrix copies
+                              and vectors alone (24 and 136) do not, gets device memory beside the
+                              pool, one such LP at a time */
   int32_t max_active;      /* LP slots (default 4096) */
   int64_t chunk_attempts;  /* attempts per LP per step for LPs with at most 16,384 nonzeros
                               per block; larger LPs get proportionally fewer (at least 8), so

@@ -387,6 +387,7 @@ struct Server {
   // the chunks of the memory cache that everything below sits in
   Chunk device_chunk, pinned_chunk, table_chunk;
   std::unique_ptr<PoolAllocator> alloc;
+  int own_chunks = 0;     // running LPs with a chunk of their own, beside the pool: at most one
   BatchSlot* d_slots = nullptr;
   NewSlot* d_fresh = nullptr;  // the LPs being admitted
   Ctrl* d_ctrls = nullptr;
@@ -840,6 +841,7 @@ static void release(Server& s, Job& J) {
   if (J.own_chunk) {
     MemoryCache::get().give_device(J.own_chunk);
     J.own_chunk = Chunk{};
+    --s.own_chunks;
   } else if (J.base) {
     s.alloc->release(J.pool_offset, J.bytes);
   }
@@ -854,10 +856,14 @@ static void admit(Server& s) {
     std::shared_ptr<Job> J = s.waiting.front();
     size_t at = 0;
     if (J->bytes > s.pool_bytes) {
-      // larger than the whole pool by its slices and scratch only: a chunk of its own
+      // larger than the whole pool by its slices and scratch only: a chunk of its own, one such LP at a time
+      if (s.own_chunks > 0) break;
       J->own_chunk = MemoryCache::get().take_device(s.cfg.device, J->bytes);
       J->base = static_cast<unsigned char*>(J->own_chunk.p);
-      if (!J->base) {
+      if (J->base) {
+        ++s.own_chunks;
+      } else {
+        if (s.running() > 0) break;  // what runs may give memory back
         s.waiting.pop_front();
         J->status = SANKHYA_PDHG_NUMERICAL_ERROR;
         J->message = "the LP does not fit the device's memory";
