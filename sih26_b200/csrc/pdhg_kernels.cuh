@@ -90,6 +90,8 @@ struct Ctrl {
   double farkas_margin;            // batched LPs: normalised margin S - M of the last test
   double primal_violation;         // report: the reported point's largest bound violation
   double quality[kQualitySlots];   // report: the reported point's quality slots (above)
+  // cluster kernel: device time of the norm estimate and start, of the evaluations, of the report
+  unsigned long long setup_ns, evaluate_ns, report_ns;
 };
 
 // SpMV work partition of one CSR matrix in permuted row order (rows sorted by length,

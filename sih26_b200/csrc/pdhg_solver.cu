@@ -401,6 +401,19 @@ struct Resident {
   double *x = nullptr, *red = nullptr, *y = nullptr;  // the report's outputs
 };
 
+// One launch of the resident kernel: to a final state (and its report) or the limits.
+template <class T>
+static void launch_resident(Level<T>& L, const Resident& rs, long long attempts, int evaluations, cudaStream_t stream) {
+  ResidentPlan plan = rs.plan, plan64 = rs.plan64;
+  double *x = rs.x, *red = rs.red, *y = rs.y;
+  void* args[] = {&L.P, &L.S, &plan, &plan64, &x, &red, &y, &attempts, &evaluations};
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t lc = resident_config(plan.cs, std::max(plan.bytes, plan64.bytes), stream, &attr);
+  SIH26_CUDA(cudaLaunchKernelExC(&lc, resident_function(sizeof(T) == 4, L.halpern), args),
+             SANKHYA_GPU_KERNEL_LAUNCH_FAILED);
+  ++g_launches;
+}
+
 template <class T>
 static Ctrl run_loop(Level<T>& L, const Resident& rs, int G, cudaStream_t stream, Ctrl* host_ctrl, int verbose,
                      int stall_checks, bool* stalled, LaunchTimer& timer) {
@@ -417,18 +430,10 @@ static Ctrl run_loop(Level<T>& L, const Resident& rs, int G, cudaStream_t stream
     const int launches = resident ? 1 : pairs;
     if (timer.on) timer.ensure(launches);
     if (resident) {
-      // an attempt of the reference operator may be turned down: the limit only keeps a launch finite
-      long long attempts = 400ll * pairs;
-      ResidentPlan plan = rs.plan, plan64 = rs.plan64;
-      double *x = rs.x, *red = rs.red, *y = rs.y;
-      void* args[] = {&L.P, &L.S, &plan, &plan64, &x, &red, &y, &attempts, &pairs};
-      cudaLaunchAttribute attr;
-      const cudaLaunchConfig_t lc = resident_config(plan.cs, std::max(plan.bytes, plan64.bytes), stream, &attr);
       if (timer.on) SIH26_CUDA(cudaEventRecord(timer.start[0], stream), SANKHYA_GPU_INIT_FAILED);
-      SIH26_CUDA(cudaLaunchKernelExC(&lc, resident_function(sizeof(T) == 4, L.halpern), args),
-                 SANKHYA_GPU_KERNEL_LAUNCH_FAILED);
+      // an attempt of the reference operator may be turned down: the limit only keeps a launch finite
+      launch_resident(L, rs, 400ll * pairs, pairs, stream);
       if (timer.on) SIH26_CUDA(cudaEventRecord(timer.stop[0], stream), SANKHYA_GPU_INIT_FAILED);
-      ++g_launches;
     }
     for (int k = 0; k < pairs && !resident; ++k) {
       void* ia[] = {&L.P, &L.S, &L.packed, &max_attempts};
@@ -1214,7 +1219,7 @@ static int solve_impl(const sankhya_pdhg_problem& prob, const sankhya_pdhg_param
 
   // the time limit counts from the start of the call, like the reference's Timer
   mark("norm estimate and A x0");
-  const double setup_seconds = seconds_since(t_start);
+  double setup_seconds = seconds_since(t_start);
   if (std::isfinite(prm.time_limit) && prm.time_limit > 0.0) {
     unsigned long long* d_now = a.zeros<unsigned long long>(1);
     read_clock_kernel<<<1, 1, 0, stream>>>(d_now);
@@ -1261,10 +1266,19 @@ static int solve_impl(const sankhya_pdhg_problem& prob, const sankhya_pdhg_param
   } ef{ev0, ev1};
 
   if (prm.verbose) {
-    if (resident)
-      std::printf("GPU PDHG: %d rows, %d columns, %lld nonzeros, one cluster of %d blocks x %d threads\n",
-                  m, n, q.nnz, rs.plan.cs, kThreads);
-    else
+    if (resident) {
+      // the norm estimate by itself, for the line below; the loop's first launch goes on from it
+      a.put(cm.ctrl, &c0, sizeof(Ctrl), stream);
+      if (mixed) launch_resident(L32, rs, 0, 0, stream);
+      else launch_resident(L64, rs, 0, 0, stream);
+      SIH26_CUDA(cudaMemcpyAsync(host_ctrl, cm.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, stream),
+                 SANKHYA_GPU_COPY_FAILED);
+      SIH26_CUDA(cudaStreamSynchronize(stream), SANKHYA_GPU_SYNC_FAILED);
+      c0 = *host_ctrl;
+      c0.setup_ns = c0.report_ns = 0;  // ahead of the loop's clock
+      std::printf("GPU PDHG: %d rows, %d columns, %lld nonzeros, one cluster of %d blocks x %d threads, ||A||_2 ~ %.4e\n",
+                  m, n, q.nnz, rs.plan.cs, kThreads, c0.spectral_norm);
+    } else
       std::printf("GPU PDHG: %d rows, %d columns, %lld nonzeros, %d blocks x %d threads, ||A||_2 ~ %.4e\n",
                   m, n, q.nnz, G, kThreads, spectral_norm);
     double prev = 0.0;
@@ -1343,6 +1357,7 @@ static int solve_impl(const sankhya_pdhg_problem& prob, const sankhya_pdhg_param
     }
   }
   SIH26_CUDA(cudaEventRecord(ev1, stream), SANKHYA_GPU_INIT_FAILED);
+  const double loop_end = seconds_since(t_start);
   if (fin.state == kDeviceError)
     throw Failure{SANKHYA_GPU_DEVICE_TIMEOUT, "a grid barrier timed out during the iteration loop"};
 
@@ -1457,6 +1472,16 @@ static int solve_impl(const sankhya_pdhg_problem& prob, const sankhya_pdhg_param
   fill_message(res, msg);
   res->dual_bound = (verifiable && cert.kind == 0) ? sense * f.dual_objective + prob.objective_offset
                                : (prob.maximize ? INFINITY : -INFINITY);
+  // The cluster kernel's launches hold the norm estimate and the report too: counted where the grid-wide
+  // kernels' are, and out of the timed iteration launches with the evaluations. Its set-up launches are not
+  // waited for, so the set-up is what the call took up to here without the loop and the report.
+  double solve_seconds = ms * 1e-3;
+  if (resident) {
+    solve_seconds = std::max(0.0, solve_seconds - 1e-9 * static_cast<double>(fin.setup_ns + fin.report_ns));
+    setup_seconds = std::max(setup_seconds, loop_end - solve_seconds - 1e-9 * static_cast<double>(fin.report_ns));
+    timer.seconds = std::max(0.0, timer.seconds - 1e-9 * static_cast<double>(fin.setup_ns + fin.evaluate_ns +
+                                                                             fin.report_ns));
+  }
   res->setup_seconds = setup_seconds;
   res->h2d_bytes = a.h2d_bytes;
   res->d2h_bytes = a.d2h_bytes;
@@ -1471,7 +1496,7 @@ static int solve_impl(const sankhya_pdhg_problem& prob, const sankhya_pdhg_param
   res->schedule[1] = sched_a.nnz_per_lane;
   res->schedule[2] = sched_at.stream_row_max;
   res->schedule[3] = sched_at.nnz_per_lane;
-  res->solve_seconds = ms * 1e-3;
+  res->solve_seconds = solve_seconds;
   res->total_seconds = seconds_since(t_start);
   return SANKHYA_GPU_SUCCESS;
 }

@@ -1379,8 +1379,19 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
                                            SideView<double>& sd64, const Team& tm,
                                            long long max_attempts, int max_evaluations) {
   Ctrl& c = ts.c;
+  // a single LP's sections by device time, kept by thread 0 of rank 0 (whose control block goes back)
+  const bool clock = kHalpern >= 0 && threadIdx.x == 0 && tm.rank == 0;
+  unsigned long long since = clock ? global_ns() : 0ull;
+  const auto spent = [&](unsigned long long& total) {
+    if (clock) {
+      const unsigned long long now = global_ns();
+      total += now - since;
+      since = now;
+    }
+  };
   if (threadIdx.x == 0) c = *S.ctrl;
   tm.sync();  // every block has started: its shared memory may be written
+  const bool setup = c.state == kSetup;
   SIH26_TEAM_MARK(-1);
   const bool halpern = kHalpern >= 0 ? kHalpern != 0 : c.halpern != 0;
   const bool outside = kOnlyL2 || (kHalpern < 0 && pl.outside != kInside);
@@ -1438,6 +1449,7 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
     tm.sync();
   }
   SIH26_TEAM_MARK(10);
+  if (setup) spent(c.setup_ns);
   long long left = max_attempts;
   int evaluations = max_evaluations;
   while (c.state == kRunning) {
@@ -1480,7 +1492,9 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
     }
     if (c.state == kNeedEval) {
       SIH26_TEAM_MARK(4);
+      if (clock) since = global_ns();
       team_evaluate(P, S, ts, tm);
+      spent(c.evaluate_ns);
       SIH26_TEAM_MARK(5);
       --evaluations;
       if (resident && c.state == kRunning) {
@@ -1496,8 +1510,11 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
     }
   }
   if (c.state == kConverged || c.state == kIterationLimit || c.state == kTimeLimit || c.state == kInfeasible ||
-      c.state == kUnbounded)
+      c.state == kUnbounded) {
+    if (clock) since = global_ns();
     team_report(P, S, x_out, red_out, y_out, ts, tm);
+    spent(c.report_ns);
+  }
   SIH26_TEAM_MARK(11);
   if (threadIdx.x == 0 && tm.rank == 0) *S.ctrl = c;
   tm.sync();
