@@ -17,7 +17,8 @@ LIBPATH = os.path.join(LIBDIR, LIBNAME)
 
 SOURCES = ["pdhg_solver.cu", "pdhg_host.cpp", "residuals_noalloc.cu", "batch_server.cu",
            "wire.cpp", "qp_solver.cu"]
-HEADERS = ["arena.cuh", "convexity.cuh", "device_cache.cuh", "device_common.cuh", "pdhg_kernels.cuh",
+HEADERS = ["arena.cuh", "convexity.cuh", "device_cache.cuh", "device_common.cuh", "entry_chunks.cuh",
+           "pdhg_kernels.cuh",
            "pdhg_host.cuh", "batch_kernels.cuh",
            "packed.cuh", "packed_host.cuh", "prep_kernels.cuh", "qp_norms.cuh",
            "resident.cuh", "resident_plan.cuh", "team_prep.cuh"]

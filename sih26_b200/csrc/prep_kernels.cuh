@@ -61,7 +61,7 @@ __global__ void gather(const int* perm, const T* src, long long len, T* dst) {
 __global__ void row_of_entry(const int* rptr, int m, int* row) {
   const int lane = threadIdx.x & 31;
   for (long long i = gtid() >> 5; i < m; i += gstride() >> 5)
-    for (int t = rptr[i] + lane; t < rptr[i + 1]; t += 32) row[t] = static_cast<int>(i);
+    for (unsigned t = rptr[i] + lane, e = rptr[i + 1]; t < e; t += 32) row[t] = static_cast<int>(i);
 }
 
 // out[s] = sum of |v| over segment s = [ptr[s], ptr[s+1]), in segment order: a warp per segment loads
@@ -70,10 +70,10 @@ __global__ void row_of_entry(const int* rptr, int m, int* row) {
 __global__ void segment_sums(const int* ptr, const double* v, int segments, double* out) {
   const int lane = threadIdx.x & 31;
   for (long long s = gtid() >> 5; s < segments; s += gstride() >> 5) {
-    const int b = ptr[s], e = ptr[s + 1];
+    const unsigned b = ptr[s], e = ptr[s + 1];  // unsigned: the batch behind the last may pass 2^31 - 1
     double acc = 0.0;
     double next = b + lane < e ? fabs(v[b + lane]) : 0.0;
-    for (int k = b; k < e; k += 32) {
+    for (unsigned k = b; k < e; k += 32) {
       const double mag = next;
       next = k + 32 + lane < e ? fabs(v[k + 32 + lane]) : 0.0;
       // past the end the batch holds zeros, which add nothing

@@ -38,12 +38,12 @@ __device__ __forceinline__ double ordered_dot(const double* a, const double* b, 
   const auto fill = [&](int c) {
     // thread 0's warp only adds
     for (int t = (int)threadIdx.x - 32; t < kChunk; t += kThreads - 32) {
-      const int j = c * kChunk + t;
+      const long long j = (long long)c * kChunk + t;
       if (t >= 0 && j < n) product[c & 1][t] = __dmul_rn(__ldcg(a + j), __ldcg(b + j));
     }
   };
   double s = 0.0;
-  const int chunks = (n + kChunk - 1) / kChunk;
+  const int chunks = n / kChunk + (n % kChunk != 0);
   if (threadIdx.x >= 32) fill(0);
   __syncthreads();
   for (int c = 0; c < chunks; ++c) {
@@ -66,7 +66,7 @@ __device__ __forceinline__ void ordered_rows(const NormMatrix& m, const double* 
   constexpr int kShort = 64;
   const int lane = threadIdx.x & 31;
   const int thread = rank * kThreads + threadIdx.x, threads = kNormTeam * kThreads;
-  for (int r = thread; r < m.rows; r += threads) {
+  for (unsigned r = thread; r < (unsigned)m.rows; r += threads) {
     const int b = __ldg(m.ptr + r), e = __ldg(m.ptr + r + 1);
     if (e - b > kShort) continue;
     double s = 0.0;
@@ -76,17 +76,18 @@ __device__ __forceinline__ void ordered_rows(const NormMatrix& m, const double* 
   }
   // every warp looks through rows of its own, a stride apart, so that long ones side by side spread
   const int warp = thread >> 5, warps = threads >> 5;
-  for (int r0 = warp; r0 < m.rows; r0 += 32 * warps) {
-    const int r = r0 + lane * warps;
-    const bool is_long = r < m.rows && __ldg(m.ptr + r + 1) - __ldg(m.ptr + r) > kShort;
+  for (unsigned r0 = warp; r0 < (unsigned)m.rows; r0 += 32 * warps) {
+    const unsigned r = r0 + lane * warps;
+    const bool is_long = r < (unsigned)m.rows && __ldg(m.ptr + r + 1) - __ldg(m.ptr + r) > kShort;
     for (unsigned todo = __ballot_sync(0xffffffffu, is_long); todo != 0u; todo &= todo - 1u) {
-      const int q = r0 + (__ffs(todo) - 1) * warps;
-      const int b = __ldg(m.ptr + q), e = __ldg(m.ptr + q + 1);
-      const auto product = [&](int k) {
+      const unsigned q = r0 + (__ffs(todo) - 1) * warps;
+      // unsigned: the batch behind the last may pass 2^31 - 1
+      const unsigned b = __ldg(m.ptr + q), e = __ldg(m.ptr + q + 1);
+      const auto product = [&](unsigned k) {
         return k < e ? __dmul_rn(__ldg(m.val + k), __ldcg(in + __ldg(m.idx + k))) : 0.0;
       };
       double s = 0.0, next = product(b + lane);
-      for (int k = b; k < e; k += 32) {
+      for (unsigned k = b; k < e; k += 32) {
         const double mine = next;
         next = product(k + 32 + lane);
         // past the end the lanes hold zeros, which add nothing
@@ -113,7 +114,7 @@ __global__ void __cluster_dims__(kNormTeam, 1, 1) __launch_bounds__(kThreads) qp
     team.sync();
     const double norm = __ldcg(r.scalar);
     if (norm <= 0.0) return;  // every block alike; the estimate stays 0
-    for (int j = thread; j < r.n; j += threads) v[j] = __ddiv_rn(__ldcg(v + j), norm);
+    for (unsigned j = thread; j < (unsigned)r.n; j += threads) v[j] = __ddiv_rn(__ldcg(v + j), norm);
     team.sync();
     ordered_rows(r.first, v, w, rank);
     team.sync();

@@ -23,6 +23,7 @@
 #include <cstdio>
 #include <string>
 
+#include "entry_chunks.cuh"
 #include "sankhya_pdhg_gpu.h"
 
 namespace sih26 {
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(kThreads, kColumnBlocksPerSm) column_kernel(sa
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double* park = terms[warp];
   cudaGridDependencySynchronize();
-  const int groups = (p.num_cols + 31) / 32;
+  const int groups = p.num_cols / 32 + (p.num_cols % 32 != 0);
   for (int g = blockIdx.x * (kThreads / 32) + warp; g < groups; g += gridDim.x * (kThreads / 32)) {
     const int j = g * 32 + lane;
     const bool mine = j < p.num_cols;
@@ -271,34 +272,36 @@ __global__ void __launch_bounds__(kThreads, kColumnBlocksPerSm) column_kernel(sa
     const int first = __shfl_sync(0xffffffffu, kb, 0);
     const int before = __shfl_up_sync(0xffffffffu, ke, 1);
     if (__all_sync(0xffffffffu, lane == 0 || before == kb)) {
-      for (int c0 = first; c0 < last; c0 += kChunk) {
-        const int c1 = c0 + kChunk < last ? c0 + kChunk : last;
+      for (int c0 = first, c1; c0 < last; c0 = c1) {
+        c1 = sih26::chunk_end<kChunk>(c0, last);
+        // the lanes' positions are unsigned: those past the range's end may lie past 2^31 - 1
+        const unsigned k0 = (unsigned)c0 + lane, end = c1;
         int row[kChunk / 32];
         double a[kChunk / 32];
 #pragma unroll
         for (int t = 0; t < kChunk / 32; ++t) {
-          const int k = c0 + lane + 32 * t;
-          row[t] = k < c1 ? p.row_indices[k] : 0;
-          a[t] = k < c1 ? p.values[k] : 0.0;
+          const unsigned k = k0 + 32 * t;
+          row[t] = k < end ? p.row_indices[k] : 0;
+          a[t] = k < end ? p.values[k] : 0.0;
         }
         double y[kChunk / 32];
 #pragma unroll
         for (int t = 0; t < kChunk / 32; ++t) {
-          const int k = c0 + lane + 32 * t;
+          const unsigned k = k0 + 32 * t;
           const bool good = (unsigned)row[t] < (unsigned)p.num_rows;
-          if (k < c1 && !good) atomicOr(v.error, 1u);
-          y[t] = k < c1 && good ? row_dual[row[t]] : 0.0;
+          if (k < end && !good) atomicOr(v.error, 1u);
+          y[t] = k < end && good ? row_dual[row[t]] : 0.0;
         }
 #pragma unroll
         for (int t = 0; t < kChunk / 32; ++t) {
-          const int k = c0 + lane + 32 * t;
+          const unsigned k = k0 + 32 * t;
           // the lane whose column holds entry k: the number of columns that end at or before k
           int owner = 0;
 #pragma unroll
           for (int step = 16; step > 0; step >>= 1)
-            if (__shfl_sync(0xffffffffu, ke, owner + step - 1) <= k) owner += step;
+            if ((unsigned)__shfl_sync(0xffffffffu, ke, owner + step - 1) <= k) owner += step;
           const double xo = __shfl_sync(0xffffffffu, xj, owner & 31);
-          if (k < c1) {
+          if (k < end) {
             if ((unsigned)row[t] < (unsigned)p.num_rows) atomicAdd(v.activity + row[t], a[t] * xo);
             park[lane + 32 * t] = a[t] * (-sense * y[t]);  // y = -sense * row_dual (pdhg.cpp:660)
           }
