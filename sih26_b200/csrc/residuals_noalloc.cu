@@ -171,11 +171,11 @@ __device__ __forceinline__ void column_range(const sankhya_pdhg_problem& p, int 
   ke = ke < kb ? kb : (ke > p.num_nonzeros ? p.num_nonzeros : ke);
 }
 
-// One column by one thread: scatters A x into `activity` and returns A'y of the column.
-__device__ inline double column_by_thread(const sankhya_pdhg_problem& p, int kb, int ke, double xj,
+// One column by one thread: scatters A x into `activity` and returns d + A'y of the column, the terms added to
+// d in order (pdhg.cpp:172-199: the cost comes first, so it cancels against them one by one).
+__device__ inline double column_by_thread(const sankhya_pdhg_problem& p, int kb, int ke, double xj, double d,
                                           double sense, const double* row_dual, double* activity,
                                           unsigned* error) {
-  double dot = 0.0;
   for (int k = kb; k < ke; ++k) {
     const int i = p.row_indices[k];
     if ((unsigned)i >= (unsigned)p.num_rows) {
@@ -184,9 +184,9 @@ __device__ inline double column_by_thread(const sankhya_pdhg_problem& p, int kb,
     }
     const double a = p.values[k];
     atomicAdd(activity + i, a * xj);
-    dot += a * (-sense * row_dual[i]);  // y = -sense * row_dual (pdhg.cpp:660)
+    d += a * (-sense * row_dual[i]);  // y = -sense * row_dual (pdhg.cpp:660)
   }
-  return dot;
+  return d;
 }
 
 // The whole check in one block, for LPs of at most kSmallRows rows whose columns and nonzeros a
@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(kSmallThreads) small_kernel(sankhya_pdhg_probl
     int kb, ke;
     column_range(p, j, kb, ke);
     const double xj = x[j], cost = sense * p.cost[j];
-    const double dot = column_by_thread(p, kb, ke, xj, sense, row_dual, activity, &error);
-    column_terms(p, j, xj, cost, cost + dot, c);
+    const double d = column_by_thread(p, kb, ke, xj, cost, sense, row_dual, activity, &error);
+    column_terms(p, j, xj, cost, d, c);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < p.num_rows; i += kSmallThreads)
@@ -261,12 +261,13 @@ __global__ void __launch_bounds__(kThreads, kColumnBlocksPerSm) column_kernel(sa
     const int j = g * 32 + lane;
     const bool mine = j < p.num_cols;
     int kb = 0, ke = 0;
-    double xj = 0.0, cost = 0.0, dot = 0.0;
+    double xj = 0.0, cost = 0.0;
     if (mine) {
       column_range(p, j, kb, ke);
       xj = x[j];
       cost = sense * p.cost[j];
     }
+    double d = cost;
     const int last = __shfl_sync(0xffffffffu, ke, (p.num_cols - g * 32 < 32 ? p.num_cols - g * 32 : 32) - 1);
     if (!mine) kb = ke = last;
     const int first = __shfl_sync(0xffffffffu, kb, 0);
@@ -308,14 +309,14 @@ __global__ void __launch_bounds__(kThreads, kColumnBlocksPerSm) column_kernel(sa
         }
         __syncwarp();
         const int b = kb > c0 ? kb : c0, e = ke < c1 ? ke : c1;
-        for (int k = b; k < e; ++k) dot += park[k - c0];
+        for (int k = b; k < e; ++k) d += park[k - c0];
         __syncwarp();
       }
     } else if (mine) {
       // column starts that are not in order: each lane reads its own column
-      dot = column_by_thread(p, kb, ke, xj, sense, row_dual, v.activity, v.error);
+      d = column_by_thread(p, kb, ke, xj, cost, sense, row_dual, v.activity, v.error);
     }
-    if (mine) column_terms(p, j, xj, cost, cost + dot, acc);
+    if (mine) column_terms(p, j, xj, cost, d, acc);
   }
   block_total<5, kThreads>(acc, kColumnMax, sh);
   if (threadIdx.x == 0) {
