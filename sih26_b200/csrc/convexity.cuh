@@ -97,9 +97,10 @@ __global__ void __launch_bounds__(kThreads, 1) convexity_kernel(ConvexityRun R) 
 #pragma unroll
       for (int j = 0; j < kPanel; ++j) {
         const double dj = d[j];
-        const double l = dj > 0.0 ? row[j] / dj : 0.0;
+        // 0 stands for a pivot within the slack; one that is not a number (inf - inf) goes on as in the reference
+        const double l = dj != 0.0 ? row[j] / dj : 0.0;
         row[j] = l;
-        if (dj > 0.0) {
+        if (dj != 0.0) {
 #pragma unroll
           for (int c = j + 1; c < kPanel; ++c) row[c] = minus_term(row[c], l, diag[c][j], dj);
         }
