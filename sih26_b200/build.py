@@ -20,7 +20,7 @@ SOURCES = ["pdhg_solver.cu", "pdhg_host.cpp", "residuals_noalloc.cu", "batch_ser
 HEADERS = ["arena.cuh", "convexity.cuh", "device_cache.cuh", "device_common.cuh", "entry_chunks.cuh",
            "pdhg_kernels.cuh",
            "pdhg_host.cuh", "batch_kernels.cuh",
-           "packed.cuh", "packed_host.cuh", "prep_kernels.cuh", "qp_norms.cuh",
+           "packed.cuh", "packed_host.cuh", "prep_kernels.cuh", "qp_norms.cuh", "quotient.cuh",
            "resident.cuh", "resident_plan.cuh", "team_prep.cuh"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -36,6 +36,7 @@
 
 #include "pdhg_host.cuh"
 #include "pdhg_kernels.cuh"
+#include "quotient.cuh"
 #include "resident_plan.cuh"
 
 namespace sih26 {
@@ -494,18 +495,6 @@ __device__ __forceinline__ void side_phase(const SideView<V>& sd, const V* g, Ep
 // (reference). Rows, FP64: both bounds, then y_0 and A x_0 (Halpern) or the running sum and two
 // buffers of A x (reference); FP32 level: yr, A xr, both bounds, then the reference operator's.
 
-// a / b for a positive b whose correctly rounded reciprocal rb is at hand: two corrections of a * rb by
-// the exact remainder give the correctly rounded quotient (P. Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", 1990, theorem 8.2), the bits of a / b, in five
-// operations. Quotients near the ends of the range, where a remainder could lose bits, are divided.
-__device__ __forceinline__ double quotient(double a, double b, double rb) {
-  double q = a * rb;
-  q = fma(fma(-q, b, a), rb, q);
-  q = fma(fma(-q, b, a), rb, q);
-  const double mag = fabs(q);
-  if (!(mag > 1e-250 && mag < 1e250)) q = a == 0.0 ? a : a / b;
-  return q;
-}
 // project() on bounds whose absent sides are infinite (effective_lower / _upper)
 __device__ __forceinline__ double clamp(double v, double lo, double hi) {
   double t = v > hi ? hi : v;
@@ -737,9 +726,9 @@ __device__ __noinline__ void team_halpern(const State<T>& S, const ResidentPlan&
   if (threadIdx.x < steps) {
     const double w = (double)(c.averaged + 1 + threadIdx.x) / (double)(c.averaged + 2 + threadIdx.x);
     ts.weight[threadIdx.x] = w;
-    ts.rweight[threadIdx.x] = 1.0 / w;
+    ts.rweight[threadIdx.x] = quotient_reciprocal(w);
   }
-  const double tau = c.eta / c.omega, sigma = c.eta * c.omega, rsigma = 1.0 / sigma;
+  const double tau = c.eta / c.omega, sigma = c.eta * c.omega, rsigma = quotient_reciprocal(sigma);
   int cur = c.cur;
   __syncthreads();
   for (int t = 0; t < steps; ++t, cur ^= 1) {
@@ -811,7 +800,7 @@ __device__ __noinline__ void team_attempt(const ResidentPlan& pl,
   // last warp, which has the fewest rows
   if (threadIdx.x == kThreads - 1) step_growth(c.iteration, ts.growth[0], ts.growth[1]);
   tm.sync();
-  TeamDual<T> ds{tm, yc, yn, sd.epi(), sd.at.stride, cur, sigma, 1.0 / sigma, c.pending, acc};
+  TeamDual<T> ds{tm, yc, yn, sd.epi(), sd.at.stride, cur, sigma, quotient_reciprocal(sigma), c.pending, acc};
   side_phase(sd, xn, ds);
   finish_attempt(ts, tm, acc);
 }
