@@ -483,9 +483,11 @@ __device__ __forceinline__ void team_phase(const SideView<V>& sd, const V* __res
     }
   }
 }
-template <class V, class Epi>
+// kStreams: the side's entries may be in global memory (the batched engine, and the norm estimate's FP64 view
+// beside an FP32 level; a single LP's own plan has none such).
+template <bool kStreams, class V, class Epi>
 __device__ __forceinline__ void side_phase(const SideView<V>& sd, const V* g, Epi& epi) {
-  if (sd.at.resident) team_phase<true>(sd, g, epi);
+  if (!kStreams || sd.at.resident) team_phase<true>(sd, g, epi);
   else team_phase<false>(sd, g, epi);
 }
 
@@ -714,7 +716,7 @@ __device__ __forceinline__ void load_epilogues(const Prob<T>& P, const State<T>&
 
 // `steps` (at most 40) Halpern steps, the last of which writes the iterates to global memory. A function
 // of its own, for its registers: the loop keeps both sides' offsets and the step constants in them.
-template <class T>
+template <class T, bool kStreams>
 __device__ __noinline__ void team_halpern(const State<T>& S, const ResidentPlan& pl, const SideView<T>& sp_,
                                           const SideView<T>& sd_, TeamShared& ts, const Team& tm_, int steps) {
   const SideView<T> sp = sp_, sd = sd_;
@@ -737,14 +739,14 @@ __device__ __noinline__ void team_halpern(const State<T>& S, const ResidentPlan&
     const double w = ts.weight[t], rw = ts.rweight[t];
     TeamPrimalHalpern<T> ps{tm, x, sp.epi(), sp.at.stride, tau, w, dump ? S.x[cur] : nullptr,
                             dump ? S.x[cur ^ 1] : nullptr, dump ? S.xt : nullptr};
-    side_phase(sp, y, ps);
+    side_phase<kStreams>(sp, y, ps);
     SIH26_TEAM_MARK(0);
     tm.sync();
     SIH26_TEAM_MARK(1);
     TeamDualHalpern<T> ds{tm, y, sd.epi(), sd.at.stride, sigma, w, rsigma, rw,
                           dump ? S.y[cur] : nullptr,
                           dump ? S.y[cur ^ 1] : nullptr, dump ? S.yt : nullptr, dump ? S.ax[cur ^ 1] : nullptr};
-    side_phase(sd, x, ds);
+    side_phase<kStreams>(sd, x, ds);
     SIH26_TEAM_MARK(2);
     tm.sync();
     SIH26_TEAM_MARK(3);
@@ -782,7 +784,7 @@ __device__ __forceinline__ void finish_attempt(TeamShared& ts, const Team& tm, d
 }
 
 // One attempt of the reference's adaptive step.
-template <class T>
+template <class T, bool kStreams>
 __device__ __noinline__ void team_attempt(const ResidentPlan& pl,
                                           const SideView<T>& sp_, const SideView<T>& sd_, TeamShared& ts,
                                           const Team& tm_) {
@@ -796,13 +798,13 @@ __device__ __noinline__ void team_attempt(const ResidentPlan& pl,
   const double tau = c.eta / c.omega, sigma = c.eta * c.omega;
   double acc[3] = {0.0, 0.0, 0.0};
   TeamPrimal<T> ps{tm, xc, xn, sp.epi(), sp.at.stride, tau, c.pending, acc};
-  side_phase(sp, yc, ps);
+  side_phase<kStreams>(sp, yc, ps);
   // the step factors depend on the iteration alone: formed beside the phases, by a thread of the
   // last warp, which has the fewest rows
   if (threadIdx.x == kThreads - 1) step_growth(c.iteration, ts.growth[0], ts.growth[1]);
   tm.sync();
   TeamDual<T> ds{tm, yc, yn, sd.epi(), sd.at.stride, cur, sigma, quotient_reciprocal(sigma), c.pending, acc};
-  side_phase(sd, xn, ds);
+  side_phase<kStreams>(sd, xn, ds);
   finish_attempt(ts, tm, acc);
 }
 
@@ -1063,7 +1065,7 @@ struct TeamStoreRow {
 // its first n doubles. With a plan in FP64 the sides are in shared memory (loaded by the caller) and v
 // and u are exchanged like the iterates; without one both live in S.xc and S.yc. The 30 steps' 60
 // phases took 330 us out of global memory on the 2,000 x 5,000 LP.
-template <class T>
+template <class T, bool kStreams>
 __device__ __noinline__ double team_power(const Prob<T>& P, const State<T>& S, int nnz, const ResidentPlan& pl,
                                           const SideView<double>& sp_, const SideView<double>& sd_, TeamShared& ts,
                                           const Team& tm_) {
@@ -1084,12 +1086,12 @@ __device__ __noinline__ double team_power(const Prob<T>& P, const State<T>& S, i
       const double length = sqrt(ts.total[0]);
       if (length == 0.0) return 1.0;
       TeamStoreRow to_u{tm, y, nullptr};
-      if (sd.at.resident) team_phase<true, true>(sd, x, to_u, 1.0 / length);
+      if (!kStreams || sd.at.resident) team_phase<true, true>(sd, x, to_u, 1.0 / length);
       else team_phase<false, true>(sd, x, to_u, 1.0 / length);
       tm.sync();
       double nx[1] = {0.0};
       TeamStoreRow to_v{tm, x, nx};
-      if (sp.at.resident) team_phase<true, true>(sp, y, to_v);
+      if (!kStreams || sp.at.resident) team_phase<true, true>(sp, y, to_v);
       else team_phase<false, true>(sp, y, to_v);
       team_part<1, 0u>(ts, 0, nx);
       team_total(ts, tm, 1, 0u);
@@ -1377,6 +1379,7 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
                                            TeamShared& ts, SideView<T>& sp, SideView<T>& sd, SideView<double>& sp64,
                                            SideView<double>& sd64, const Team& tm,
                                            long long max_attempts, int max_evaluations) {
+  constexpr bool kStreams = kHalpern < 0;
   Ctrl& c = ts.c;
   if (threadIdx.x == 0) c = *S.ctrl;
   if constexpr (kHalpern >= 0) section_begins(ts, tm);
@@ -1397,9 +1400,9 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
     if constexpr (kHalpern < 0) {
       norm = turns     ? vector_setup<true>(P, S, nnz, ts, tm)
              : outside ? vector_setup<false>(P, S, nnz, ts, tm)
-                       : team_power(P, S, nnz, pl64, sp64, sd64, ts, tm);
+                       : team_power<T, kStreams || kDelta<T>>(P, S, nnz, pl64, sp64, sd64, ts, tm);
     } else {
-      norm = team_power(P, S, nnz, pl64, sp64, sd64, ts, tm);
+      norm = team_power<T, kStreams || kDelta<T>>(P, S, nnz, pl64, sp64, sd64, ts, tm);
     }
     if (threadIdx.x == 0) {
       c.spectral_norm = norm;
@@ -1430,7 +1433,7 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
       if constexpr (!kDelta<T>) {
         // A x_0 with the iteration's sums; also the Halpern anchor's
         TeamStoreAx st{S.ax[c.cur], S.axr};
-        side_phase(sd, reinterpret_cast<const T*>(team_memory() + pl.x[c.cur]), st);
+        side_phase<kStreams>(sd, reinterpret_cast<const T*>(team_memory() + pl.x[c.cur]), st);
         __syncthreads();
       }
       if (threadIdx.x == 0) c.state = kRunning;
@@ -1459,7 +1462,7 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
       if (steps > c.iteration_limit - c.iteration) steps = c.iteration_limit - c.iteration;
       if (steps > left) steps = left;
       if (resident) {
-        team_halpern(S, pl, sp, sd, ts, tm, static_cast<int>(steps));
+        team_halpern<T, kStreams>(S, pl, sp, sd, ts, tm, static_cast<int>(steps));
       } else {
         if constexpr (kHalpern < 0) {
           if (turns) vector_halpern<true>(P, S, ts, tm, static_cast<int>(steps));
@@ -1470,7 +1473,7 @@ __device__ __forceinline__ void team_solve(const Prob<T>& P, const State<T>& S, 
     } else {
       do {
         if (resident) {
-          team_attempt(pl, sp, sd, ts, tm);
+          team_attempt<T, kStreams>(pl, sp, sd, ts, tm);
         } else {
           if constexpr (kHalpern < 0) {
             if (turns) vector_attempt<true>(P, S, ts, tm);
