@@ -703,20 +703,36 @@ int clusters_for_round(const Server& s, long long small_nnz, long long big_nnz, 
   return std::max(1, want);
 }
 
-// Of them, those for the LPs gathered out of L2: as many as there are where every large LP has a cluster, else
-// their share of the large LPs' nonzeros, at least one and one less than all where there are others. Rounded up:
-// an LP that waits for a cluster takes a round twice as long, and these have the longest.
-int l2_clusters_for_round(const Server& s, int clusters, long long big_nnz, long long l2_nnz) {
-  const int count = static_cast<int>(s.cls[kClusterL2].active.size());
-  const int others = static_cast<int>(s.cls[kCluster].active.size());
-  if (count == 0) return 0;
-  if (others == 0) return clusters;
-  if (count + others <= clusters) return count;
-  const double share = static_cast<double>(l2_nnz) / static_cast<double>(std::max(1ll, big_nnz));
-  const int want = std::max(1, std::min({count, clusters - 1, static_cast<int>(std::ceil(share * clusters))}));
-  // hysteresis: a few too many are not worth a new graph
-  const int now = s.l2_clusters;
-  return now >= want && now - want <= now / 4 && now < clusters && now <= count ? now : want;
+// Of them, those for the LPs gathered out of L2: the split with the shortest round. An LP's share of a round goes
+// with its nonzeros up to the chunk's budget (run_slot), which all larger ones take in full; a class lasts as
+// long as its LPs take side by side, and as its largest take in turns. (Split by nonzeros alone, a queue of the
+// served family left the smaller clusters' LPs a third of the clusters that they needed.)
+int l2_clusters_for_round(const Server& s, int clusters) {
+  const double budget = s.chunk > 0 ? static_cast<double>(kChunkNnz) * kClusterSize : INFINITY;
+  double total[kKinds] = {0, 0, 0}, top[kKinds] = {0, 0, 0};
+  int count_top[kKinds] = {0, 0, 0};
+  for (int k = kCluster; k < kKinds; ++k)
+    for (int slot : s.cls[k].active) {
+      const double w = std::min(budget, static_cast<double>(s.slot_job[slot]->nnz));
+      total[k] += w;
+      if (w > top[k]) count_top[k] = 0;
+      top[k] = std::max(top[k], w);
+      count_top[k] += w == top[k];
+    }
+  if (s.cls[kClusterL2].active.empty()) return 0;
+  if (s.cls[kCluster].active.empty()) return clusters;
+  const auto lasts = [&](int k, int c) { return std::max(total[k] / c, top[k] * ((count_top[k] + c - 1) / c)); };
+  int best = 1;
+  double best_time = INFINITY;
+  for (int l2 = 1; l2 < clusters; ++l2) {
+    const double time = std::max(lasts(kClusterL2, l2), lasts(kCluster, clusters - l2));
+    // of equal ones the present split, which needs no new graph
+    if (time < best_time || (time == best_time && l2 == s.l2_clusters)) {
+      best = l2;
+      best_time = time;
+    }
+  }
+  return best;
 }
 
 // Bytes of the report's outputs, from off.xc on.
@@ -1007,7 +1023,7 @@ static void run_round(Server& s) {
   // hysteresis, as above
   if (s.graph && std::abs(want - s.clusters) <= std::max(1, s.clusters / 4)) want = s.clusters;
   want = std::max(1, std::min(want, s.max_clusters));
-  const int l2 = l2_clusters_for_round(s, want, big_nnz, nnz[kClusterL2]);
+  const int l2 = l2_clusters_for_round(s, want);
   // a class with LPs always gets a cluster (one that does not fit beside the others waits for them)
   build_graph(s, std::max(want - l2, s.cls[kCluster].active.empty() ? 0 : 1), l2);
   for (Server::Class& c : s.cls) {
