@@ -1069,7 +1069,7 @@ void sankhya_pdhg_server_default_config(sankhya_pdhg_server_config* c) {
   c->chunk_attempts = -1;  // the autotuner's (measured against fixed lengths on the served family)
   c->cluster_min_nnz = 16384;
   c->clusters = 0;  // adaptive: the large class's share of the active nonzeros
-  c->solo_min_nnz = 0;  // never: routing measured slower on the served family
+  c->solo_min_nnz = 0;  // never: routing gains nothing on the served family
 }
 
 int sankhya_pdhg_server_create(const sankhya_pdhg_server_config* config,
