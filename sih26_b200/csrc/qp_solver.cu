@@ -237,6 +237,15 @@ device_error:
 // 2.8 and 3.7, 320,000 18.8 and 27.1, 520,000 26 and 42; two entries 0.47 and 0.31.
 constexpr long long kDeviceNorms = 20000;
 
+// Unless a row or column holds most of it: its ordered sum is one warp's chain of loads and additions, 18 ns an
+// entry (a vector's 4), against the host's 1.3 an operation. A solve on the device and here, in ms: one row of 20,000
+// with a diagonal Q 10.3 and 6.0, of 200,000 104 and 65; 10 rows of 200,000 128 and 124, 100 of some 1,000 21 and 53.
+bool norms_on_device(int n, long long nnz_a, long long nnz_q, int longest) {
+  const double device_ns = 18.0 * longest + 4.0 * n;
+  const double host_ns = 1.3 * (2.0 * static_cast<double>(nnz_a) + static_cast<double>(nnz_q) + 2.0 * n);
+  return nnz_a + nnz_q >= kDeviceNorms && device_ns < host_ns;
+}
+
 // The reference's spectral_norm (qp_condat_vu.cpp:64-97): 20 power iterations on A'A from
 // mt19937(26119) uniform(-1, 1), multiply_add / transpose_multiply_add in their order.
 double qp_norm_a(const sankhya_pdhg_problem& p) {
@@ -541,7 +550,11 @@ int qp_solve_impl(const sankhya_pdhg_problem& prob, const sankhya_qp_hessian& he
 
   // ---- norm estimates: on the device beside the layout, or here. The sign of Q_s cancels. ----
   double norms[2] = {0.0, 0.0};
-  const bool device_norms = prob.num_nonzeros + static_cast<long long>(q_ptr[n]) >= kDeviceNorms;
+  int longest = 0;
+  for (int i = 0; i < m; ++i) longest = std::max(longest, rlen[i]);
+  for (int j = 0; j < n; ++j)
+    longest = std::max({longest, prob.col_starts[j + 1] - prob.col_starts[j], q_ptr[j + 1] - q_ptr[j]});
+  const bool device_norms = norms_on_device(n, prob.num_nonzeros, q_ptr[n], longest);
   double* d_scalars = nullptr;
   if (device_norms) {
     const bool has_a = m > 0 && n > 0 && prob.num_nonzeros > 0, has_q = hes.num_nonzeros > 0 && n > 0;
