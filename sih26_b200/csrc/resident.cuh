@@ -823,6 +823,7 @@ __device__ __forceinline__ void turn_phase(const Csr<double>& M, const Part& p, 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ib = __ldg(p.blk_item_begin + rank), ie = __ldg(p.blk_item_begin + rank + 1);
   const int lb = __ldg(p.blk_long_begin + rank), le = __ldg(p.blk_long_begin + rank + 1);
+  const int sb = __ldg(p.blk_seg_begin + rank), se = __ldg(p.blk_seg_begin + rank + 1);
   const int* __restrict__ sidx = p.sell_idx;
   const double* __restrict__ sval = static_cast<const double*>(p.sell_val);
   const auto add = [&](double s, double a, double x) {
@@ -846,16 +847,19 @@ __device__ __forceinline__ void turn_phase(const Csr<double>& M, const Part& p, 
     if ((size & 1) && threadIdx.x == 0) g[size - 1] = kRound ? vec[size - 1] * scale : vec[size - 1];
   }
   __syncthreads();
-  for (int q = lb + warp; q < le; q += kWarps) {  // long rows: a warp each
-    const int r = __ldg(p.longs + q).x, b = __ldg(M.ptr + r), e = __ldg(M.ptr + r + 1);
-    typename Epi::In in{};
-    if (lane == 0) in = epi.load(r);
-    double s[1] = {0.0};
-#pragma unroll 4
-    for (int k = b + lane; k < e; k += 32) s[0] += __ldg(M.val64 + k) * g[__ldg(M.idx + k)];
+  // long rows in segments, a warp each, folded at the end (a warp for a whole row of 20,000 took 46 us an
+  // iteration where the segments take 23)
+  for (int q = sb + warp; q < se; q += kWarps) {
+    const int4 sg = __ldg(p.segs + q);
+    double s = 0.0;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
-    if (lane == 0) epi.apply(r, s, in, acc);
+    for (int t = 0; t < kSegment / 32; ++t) {
+      const int k = sg.y + lane + 32 * t;
+      if (k < sg.z) s += __ldg(M.val64 + k) * g[__ldg(M.idx + k)];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane == 0) p.seg_sum[q] = s;
   }
   // the headers of the warp's next rows are on their way while these are summed: the item two
   // ahead, its rows' range one ahead
@@ -915,6 +919,19 @@ __device__ __forceinline__ void turn_phase(const Csr<double>& M, const Part& p, 
     item = next;
     next = after;
     h = hn;
+  }
+  if (le > lb) {
+    __syncthreads();
+    for (int q = lb + warp; q < le; q += kWarps) {
+      const int4 lr = __ldg(p.longs + q);
+      typename Epi::In in{};
+      if (lane == 0) in = epi.load(lr.x);
+      double s[1] = {0.0};
+      for (int k = lane; k < lr.z; k += 32) s[0] += p.seg_sum[lr.y + k];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
+      if (lane == 0) epi.apply(lr.x, s, in, acc);
+    }
   }
 }
 
